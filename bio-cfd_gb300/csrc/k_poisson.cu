@@ -44,14 +44,71 @@ struct DivOp {
   }
 };
 
-// rhs = b / deltat, once per solve (the reference divides inside every sweep;
-// the quotient is the same IEEE value)
-__global__ void k_rhs(DevBlock B, double dt) {
-  const int64_t n = B.d.npacked();
+// v / d, correctly rounded, from the stored reciprocal s of a negative d
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990: with y = RN(1/d) and q within one ulp
+// of v/d, RN(q + y (v - d q)) is RN(v/d); the remainder is exact by FMA).
+// q0 = RN(v y) is off by at most half an ulp plus |v/d| |1 - d y|, which is
+// within one ulp where |1 - d y| <= 2^-54; elsewhere (s > 0) a first
+// correction brings it there.  Holds while no intermediate leaves the normal
+// range: |d| in (kDivMin, kDivMax) by k_rhs, |v| tested here (and v = 0, whose
+// quotient's sign the three steps keep for a negative d); everything else
+// (tiny or huge v, Inf, NaN, a diagonal out of range) takes the division.
+// Three or five FP64 instructions, against the division's ten-odd.
+constexpr double kDivMin = 0x1p-300, kDivMax = 0x1p300;
+__device__ __noinline__ double ieee_div(double v, double d) { return v / d; }
+__device__ __forceinline__ double div_by(double v, double d, double s) {
+  const int sh = __double2hiint(s);
+  const double y = __hiloint2double(sh | (int)0x80000000, __double2loint(s));
+  double q = v * y;
+  q = fma(fma(-q, d, v), y, q);
+  const unsigned vh = (unsigned)__double2hiint(v) & 0x7fffffffu;
+  const bool usual = vh - 0x2d300000u < 0x25800000u || (vh | (unsigned)__double2loint(v)) == 0u;
+  if (sh >= 0) q = fma(fma(-q, d, v), y, q);
+  if (!usual || (sh & 0x7ff00000) == 0x7ff00000) q = ieee_div(v, d);
+  return q;
+}
+
+// What the FP64 sweeps of one solve read beside pc, per updated cell:
+//  * rhs = b / deltat (the reference divides inside every sweep; the quotient
+//    is the same IEEE value);
+//  * dg = (ax2 + ay2) + az2, the diagonal, in the reference's order;
+//  * dgi: with `fast`, omega times the reciprocal of the diagonal (an FP32
+//    reciprocal refined by one Newton-Raphson step, y1 = y0 + y0 (1 - d y0));
+//    else the correctly rounded reciprocal y = 1/dg that div_by takes, stored
+//    with its sign cleared where div_by needs its second correction and as
+//    NaN where dg is out of the range its proof covers.
+// One pass per solve (one division per cell) replaces an addition pair and a
+// division in every one of the solve's hundreds of updates per cell: GB300
+// issues FP64 at 1/64 of the FP32 rate, so the FP64 sweeps are bound by their
+// count of FP64 instructions (memory is at 10-15% of its rate).
+__global__ void k_rhs(DevBlock B, double dt, double omega, int fast) {
+  const Dims& d = B.d;
+  const int64_t n = d.npacked();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x) {
-    B.rhs[0][t] = B.bpk[0][t] / dt;
-    B.rhs[1][t] = B.bpk[1][t] / dt;
+    const int h = (int)(t % d.NXH);
+    const int64_t r = t / d.NXH;
+    const int j = 1 + (int)(r % d.NY), k = 1 + (int)(r / d.NY);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      B.rhs[c][t] = B.bpk[c][t] / dt;
+      if (!B.upd[c][t]) continue;
+      const int i = 2 * h + 1 + (((1 + j + k) & 1) != c);
+      const double dg = B.Acx[i - 2 + d.nx] + B.Acy[j - 2 + d.ny] + B.Acz[k - 2 + d.nz];
+      double y;
+      if (fast) {
+        const double y0 = (double)__frcp_rn((float)dg);
+        y = omega * fma(y0, fma(-dg, y0, 1.0), y0);
+      } else if (dg < -kDivMin && dg > -kDivMax) {
+        y = 1.0 / dg;
+        if (fabs(fma(-dg, y, 1.0)) > 0x1p-54) y = -y;
+      } else {
+        y = __longlong_as_double(0x7ff8000000000000ll);
+      }
+      B.dg[c][t] = dg;
+      B.dgi[c][t] = y;
+    }
   }
 }
 
@@ -73,6 +130,10 @@ __global__ void k_rhs(DevBlock B, double dt) {
 // largest CTA of the FP64 tiled solve, and the FP32 solve's largest CTA (its
 // four-cell runs need ~80 registers: three CTAs of 256 threads per SM)
 constexpr int kSolveMaxThreads = 512;
+// default of the FP64 solve: three CTAs of 256 threads per SM, within 7% of one
+// of 512 on large blocks and 15-25% faster on blocks up to 64^3 (a tile's tail
+// idles fewer warps)
+constexpr int kSor64Threads = 256;
 constexpr int kDcThreads = 256;
 
 struct TileMap {
@@ -176,77 +237,86 @@ __device__ __forceinline__ Pos tile_pos(const DevBlock& B, const Tile& t, const 
   return p;
 }
 
-// reference SOR update of one FP64 cell (no FMA; the expression order of
-// src/PcorVcor.F90:319-327); `old` returns the previous value
-template <int C>
-__device__ __forceinline__ double sor64_cell(const DevBlock& B, const Pos& p, double omega, double& old) {
+// (bound by the FP64 pipe: 20-23 FP64 instructions per update against 29 with
+// the division and the diagonal's sum in every update, 8 against 17 with FAST;
+// 384x256x256: 2063 -> 1017 us per sweep pair, FAST 920 -> 389 us; 128x96x96:
+// 108 -> 58 and 52 -> 25 us)
+// One FP64 half-sweep of colour C over the tile, two consecutive packed cells
+// per thread (double2 loads as in tile_residual64v).  FAST = 0: the
+// reference's update (no FMA, the expression order of src/PcorVcor.F90:319-327,
+// its division by div_by: the same bits); 1: without a division, for solves
+// that stop on the FP64 residual (precision 3), r = b/dt - A pc by fused
+// multiply-adds, then x + (omega/d) r with omega/d from k_rhs; its fixed point
+// A x = b does not depend on that factor's rounding.  CHK: lmax takes
+// max |new - old| as a bit pattern (of non-negative numbers: ordered as
+// integers, NaN above everything), needed only by the half-sweeps before the
+// reference's stop test.
+template <int C, int FAST, int CHK>
+__device__ __forceinline__ void tile_half64(const DevBlock& B, const Tile& t, double omega,
+                                            unsigned long long& lmax) {
   const Dims& d = B.d;
-  const double* __restrict__ o = B.pc[1 - C];
-  const int64_t sy = d.NXH, sz = (int64_t)d.NXH * d.NY;
-  const int i = p.ic, j = p.j, k = p.k, nx = d.nx, ny = d.ny, nz = d.nz;
-  // values written by other CTAs in this launch: read through L2 (ld.cg)
-  const double pl = __ldcg(o + p.row + ((p.i - 2) >> 1));
-  const double pr = __ldcg(o + p.row + (p.i >> 1));
-  const double ps = __ldcg(o + p.pi - sy), pn = __ldcg(o + p.pi + sy);
-  const double pb = __ldcg(o + p.pi - sz), pt = __ldcg(o + p.pi + sz);
-  old = __ldcg(B.pc[C] + p.pi);
-  const double ax1 = B.Acx[i - 2], ax2 = B.Acx[i - 2 + nx], ax3 = B.Acx[i - 2 + 2 * nx];
-  const double ay1 = B.Acy[j - 2], ay2 = B.Acy[j - 2 + ny], ay3 = B.Acy[j - 2 + 2 * ny];
-  const double az1 = B.Acz[k - 2], az2 = B.Acz[k - 2 + nz], az3 = B.Acz[k - 2 + 2 * nz];
-  double v = B.rhs[C][p.pi] - ax1 * pl - ax3 * pr - ay1 * ps - ay3 * pn - az1 * pb - az3 * pt;
-  v = v / (ax2 + ay2 + az2);
-  return (1.0 - omega) * old + omega * v;
-}
-
-// One half-sweep of colour C over the tile, FP64, reference arithmetic; one
-// cell per pass (the FP64 sweep is bound by the FP64 divide, and the lower
-// register count keeps two CTAs of 512 threads per SM)
-// SOR update of one FP64 cell without a division, for solves that stop on
-// the FP64 residual (precision 3): r = b/dt - A_offdiag pc by fused
-// multiply-adds, then x + omega r / d.  1/d is an FP32 reciprocal refined by
-// one Newton-Raphson step in FP64 (y1 = y0 + y0 (1 - d y0)), accurate to a
-// few FP64 ulps; the iteration's fixed point A x = b does not depend on it.
-template <int C>
-__device__ __forceinline__ double sor64f_cell(const DevBlock& B, const Pos& p, double omega, double& old) {
-  const Dims& d = B.d;
-  const double* __restrict__ o = B.pc[1 - C];
-  const int64_t sy = d.NXH, sz = (int64_t)d.NXH * d.NY;
-  const int i = p.ic, j = p.j, k = p.k, nx = d.nx, ny = d.ny, nz = d.nz;
-  const double pl = __ldcg(o + p.row + ((p.i - 2) >> 1));
-  const double pr = __ldcg(o + p.row + (p.i >> 1));
-  const double ps = __ldcg(o + p.pi - sy), pn = __ldcg(o + p.pi + sy);
-  const double pb = __ldcg(o + p.pi - sz), pt = __ldcg(o + p.pi + sz);
-  old = __ldcg(B.pc[C] + p.pi);
-  const double ax1 = B.Acx[i - 2], ax2 = B.Acx[i - 2 + nx], ax3 = B.Acx[i - 2 + 2 * nx];
-  const double ay1 = B.Acy[j - 2], ay2 = B.Acy[j - 2 + ny], ay3 = B.Acy[j - 2 + 2 * ny];
-  const double az1 = B.Acz[k - 2], az2 = B.Acz[k - 2 + nz], az3 = B.Acz[k - 2 + 2 * nz];
-  const double dg = ax2 + ay2 + az2;
-  double r = fma(-dg, old, B.rhs[C][p.pi]);
-  r = fma(-ax1, pl, r);
-  r = fma(-ax3, pr, r);
-  r = fma(-ay1, ps, r);
-  r = fma(-ay3, pn, r);
-  r = fma(-az1, pb, r);
-  r = fma(-az3, pt, r);
-  const double y0 = (double)__frcp_rn((float)dg);
-  const double y1 = fma(y0, fma(-dg, y0, 1.0), y0);
-  return fma(omega * y1, r, old);
-}
-
-template <int C>
-__device__ __forceinline__ void tile_half64(const DevBlock& B, const Tile& t, double omega, double& lmax,
-                                            int fast) {
   double* __restrict__ own = B.pc[C];
-  const int n = B.d.NXH * t.nj * t.nk;
+  const double* __restrict__ o = B.pc[1 - C];
+  const double* __restrict__ rhs = B.rhs[C];
+  const double* __restrict__ dgp = B.dg[C];
+  const double* __restrict__ dip = B.dgi[C];
+  const uint8_t* __restrict__ upd = B.upd[C];
+  const int nh = d.NXH >> 1, nx = d.nx, ny = d.ny, nz = d.nz;
+  const int64_t sy = d.NXH, sz = (int64_t)d.NXH * d.NY;
+  const int n = nh * t.nj * t.nk;
+  const double om1 = 1.0 - omega;
   Walk3 w;
-  w.init(threadIdx.x, blockDim.x, B.d.NXH, t.nj);
+  w.init(threadIdx.x, blockDim.x, nh, t.nj);
   for (int q = threadIdx.x; q < n; q += blockDim.x, w.next()) {
-    const Pos p = tile_pos<C>(B, t, w, true);
-    if (!p.on) continue;
-    double old;
-    const double nv = fast ? sor64f_cell<C>(B, p, omega, old) : sor64_cell<C>(B, p, omega, old);
-    own[p.pi] = nv;
-    lmax = nmax(lmax, fabs(nv - old));
+    const int h0 = 2 * w.a, j = t.j0 + w.b, k = t.k0 + w.c;
+    const int64_t pi = (int64_t)d.NXH * (j - 1) + sz * (k - 1) + h0;
+    const uchar2 mk = *reinterpret_cast<const uchar2*>(upd + pi);
+    if (!(mk.x | mk.y)) continue;
+    const int par = ((1 + j + k) & 1) != C;
+    const double2 oc = *reinterpret_cast<const double2*>(o + pi);
+    const double2 os = *reinterpret_cast<const double2*>(o + pi - sy);
+    const double2 on = *reinterpret_cast<const double2*>(o + pi + sy);
+    const double2 ob = *reinterpret_cast<const double2*>(o + pi - sz);
+    const double2 ot = *reinterpret_cast<const double2*>(o + pi + sz);
+    const double2 x2 = *reinterpret_cast<const double2*>(own + pi);
+    const double2 b2 = *reinterpret_cast<const double2*>(rhs + pi);
+    const double2 d2 = *reinterpret_cast<const double2*>(dgp + pi);
+    const double2 s2 = *reinterpret_cast<const double2*>(dip + pi);
+    const double ox = par ? o[pi + 2] : o[pi - 1];
+    const double ay1 = B.Acy[j - 2], ay3 = B.Acy[j - 2 + 2 * ny];
+    const double az1 = B.Acz[k - 2], az3 = B.Acz[k - 2 + 2 * nz];
+    double nv[2] = {x2.x, x2.y};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const double left = u == 0 ? (par ? oc.x : ox) : (par ? oc.y : oc.x);
+      const double right = u == 0 ? (par ? oc.y : oc.x) : (par ? ox : oc.y);
+      // i clamped to the interior (a cell that is not updated may sit outside)
+      const int ic = min(max(2 * (h0 + u) + 1 + par, 2), nx + 1);
+      const double ax1 = B.Acx[ic - 2], ax3 = B.Acx[ic - 2 + 2 * nx];
+      const double old = nv[u], dg = u == 0 ? d2.x : d2.y, si = u == 0 ? s2.x : s2.y;
+      const double ps = u == 0 ? os.x : os.y, pn = u == 0 ? on.x : on.y;
+      const double pb = u == 0 ? ob.x : ob.y, pt = u == 0 ? ot.x : ot.y;
+      double v = u == 0 ? b2.x : b2.y;
+      if (FAST) {
+        v = fma(-dg, old, v);
+        v = fma(-ax1, left, v);
+        v = fma(-ax3, right, v);
+        v = fma(-ay1, ps, v);
+        v = fma(-ay3, pn, v);
+        v = fma(-az1, pb, v);
+        v = fma(-az3, pt, v);
+        v = fma(si, v, old);
+      } else {
+        v = v - ax1 * left - ax3 * right - ay1 * ps - ay3 * pn - az1 * pb - az3 * pt;
+        v = om1 * old + omega * div_by(v, dg, si);
+      }
+      if (u == 0 ? mk.x : mk.y) {
+        nv[u] = v;
+        if (CHK) lmax = max(lmax, (unsigned long long)__double_as_longlong(fabs(v - old)));
+      }
+    }
+    // cells that are not updated keep their value; no other CTA writes them
+    *reinterpret_cast<double2*>(own + pi) = make_double2(nv[0], nv[1]);
   }
 }
 
@@ -259,10 +329,10 @@ __device__ __forceinline__ double resid64_cell(const DevBlock& B, const Pos& p) 
   const double* __restrict__ o = B.pc[1 - C];
   const int64_t sy = d.NXH, sz = (int64_t)d.NXH * d.NY;
   const int i = p.ic, j = p.j, k = p.k;
-  const double ax1 = B.Acx[i - 2], ax2 = B.Acx[i - 2 + d.nx], ax3 = B.Acx[i - 2 + 2 * d.nx];
-  const double ay1 = B.Acy[j - 2], ay2 = B.Acy[j - 2 + d.ny], ay3 = B.Acy[j - 2 + 2 * d.ny];
-  const double az1 = B.Acz[k - 2], az2 = B.Acz[k - 2 + d.nz], az3 = B.Acz[k - 2 + 2 * d.nz];
-  double ax = (ax2 + ay2 + az2) * __ldcg(own + p.pi);
+  const double ax1 = B.Acx[i - 2], ax3 = B.Acx[i - 2 + 2 * d.nx];
+  const double ay1 = B.Acy[j - 2], ay3 = B.Acy[j - 2 + 2 * d.ny];
+  const double az1 = B.Acz[k - 2], az3 = B.Acz[k - 2 + 2 * d.nz];
+  double ax = B.dg[C][p.pi] * __ldcg(own + p.pi);
   ax = fma(ax1, __ldcg(o + p.row + ((p.i - 2) >> 1)), ax);
   ax = fma(ax3, __ldcg(o + p.row + (p.i >> 1)), ax);
   ax = fma(ay1, __ldcg(o + p.pi - sy), ax);
@@ -352,6 +422,26 @@ __device__ __forceinline__ double take_slot(BlockStats* st, int c, int cta) {
   return v;
 }
 
+// one half-sweep of the pair's first (FIRST = 1: red, or black for the
+// adjoint's order) or second colour
+template <int FIRST>
+__device__ __forceinline__ void sor64_half(const DevBlock& B, const Tile& t, const SorArgs& a, bool chk,
+                                           unsigned long long& lmax) {
+  if (a.fast && chk) {
+    if (a.rev) tile_half64<1 - FIRST, 1, 1>(B, t, a.omega, lmax);
+    else tile_half64<FIRST, 1, 1>(B, t, a.omega, lmax);
+  } else if (a.fast) {
+    if (a.rev) tile_half64<1 - FIRST, 1, 0>(B, t, a.omega, lmax);
+    else tile_half64<FIRST, 1, 0>(B, t, a.omega, lmax);
+  } else if (chk) {
+    if (a.rev) tile_half64<1 - FIRST, 0, 1>(B, t, a.omega, lmax);
+    else tile_half64<FIRST, 0, 1>(B, t, a.omega, lmax);
+  } else {
+    if (a.rev) tile_half64<1 - FIRST, 0, 0>(B, t, a.omega, lmax);
+    else tile_half64<FIRST, 0, 0>(B, t, a.omega, lmax);
+  }
+}
+
 // REDBLACKSOR_linear (src/PcorVcor.F90:288-377) as one cooperative launch.
 // nIterPcor continues from stats->niter (the fine blocks accumulate it over
 // two solves per step, :78, :98, :116) and the stop test runs whenever the
@@ -382,16 +472,15 @@ __device__ __forceinline__ void sor64_body(const DevBlock& B, const SorArgs& a, 
   for (;;) {
     ++it;
     if (++r5 == 5) r5 = 0;
-    double lmax = 0.0;
+    unsigned long long lbits = 0;
     if (!tile_wait(tm, gb, t, ph)) { ok = false; break; }
-    if (a.rev) tile_half64<0>(B, t, a.omega, lmax, a.fast);
-    else tile_half64<1>(B, t, a.omega, lmax, a.fast);
+    sor64_half<1>(B, t, a, !target_mode && r5 == 0, lbits);
     tile_publish(tm, t, ++ph);
     if (!tile_wait(tm, gb, t, ph)) { ok = false; break; }
-    if (a.rev) tile_half64<1>(B, t, a.omega, lmax, a.fast);
-    else tile_half64<0>(B, t, a.omega, lmax, a.fast);
+    sor64_half<0>(B, t, a, !target_mode && r5 == 0, lbits);
     tile_publish(tm, t, ++ph);
     if (target_mode ? it >= next_check : r5 == 0) {
+      double lmax = __longlong_as_double((long long)lbits);
       if (target_mode) {
         // residual-target mode: the residual needs the neighbours' sweep pair
         if (!tile_wait(tm, gb, t, ph)) { ok = false; break; }
@@ -682,7 +771,9 @@ __device__ __forceinline__ void sor_dc_body(const DevBlock& B, const DcArgs& a, 
   }
 }
 
-__global__ void __launch_bounds__(kSolveMaxThreads, 2) k_sor64(DevBlock B, SorArgs a, GridBar gb, TileMap tm) {
+// NT threads at most: 256 (80 registers, three CTAs per SM) or 512 (one CTA)
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 3 : 1) k_sor64(DevBlock B, SorArgs a, GridBar gb, TileMap tm) {
   sor64_body(B, a, gb, tm, (int)blockIdx.x);
 }
 
@@ -1347,7 +1438,7 @@ __device__ __forceinline__ int solve_member(const SolveSet<Args>& S) {
   return m;
 }
 
-__global__ void __launch_bounds__(kSolveMaxThreads, 2) k_sor64_set(SolveSet<SorArgs> S) {
+__global__ void __launch_bounds__(256, 3) k_sor64_set(SolveSet<SorArgs> S) {
   __shared__ unsigned long long raw[(sizeof(DevBlock) + 7) / 8];
   const int m = solve_member(S);
   BlockSet bs;
@@ -1642,13 +1733,36 @@ static int reset_solve_state(HostBlock* hb, const TileMap& tm) {
   return 0;
 }
 
+// the FP64 sweeps' diagonal arrays (the first FP64 solve of a block)
+static int ensure_diag(HostBlock* hb) {
+  if (hb->d.dg[0]) return 0;
+  const size_t np = (size_t)hb->d.d.npacked();
+  void* p = nullptr;
+  if (cudaMalloc(&p, 4 * np * sizeof(double)) != cudaSuccess) return BCFD_E_NOMEM;
+  hb->allocs.push_back(p);
+  // cells that are not updated are read (two cells per thread) but not used
+  BCFD_CUDA(cudaMemsetAsync(p, 0, 4 * np * sizeof(double), stream()));
+  double* q = static_cast<double*>(p);
+  for (int c = 0; c < 2; ++c) {
+    hb->d.dg[c] = q + c * np;
+    hb->d.dgi[c] = q + (2 + c) * np;
+  }
+  return 0;
+}
+
+static int launch_rhs(HostBlock* hb, double dt, int fast) {
+  TRY_R(ensure_diag(hb));
+  k_rhs<<<grid_for(hb->d.d.npacked(), 256), 256, 0, stream()>>>(hb->d, dt, hb->omega, fast);
+  BCFD_LAUNCHED();
+  return 0;
+}
+
 int launch_sor(HostBlock* hb, int64_t itmax, double dt, double epsi, double res_tol, int fast) {
   DevBlock& B = hb->d;
-  const int64_t np = B.d.npacked();
-  k_rhs<<<grid_for(np, 256), 256, 0, stream()>>>(B, dt);
-  BCFD_LAUNCHED();
-  const int threads = hb->solve_threads > 0 ? hb->solve_threads : 512;
-  TileMap tm = choose_tiles(hb, (const void*)k_sor64, threads, hb->solve_sync == 1 ? 1 : 0, hb->solve_ctas_per_sm);
+  TRY_R(launch_rhs(hb, dt, fast));
+  const int threads = hb->solve_threads > 0 ? hb->solve_threads : kSor64Threads;
+  const void* fn = threads > 256 ? (const void*)k_sor64<kSolveMaxThreads> : (const void*)k_sor64<256>;
+  TileMap tm = choose_tiles(hb, fn, threads, hb->solve_sync == 1 ? 1 : 0, hb->solve_ctas_per_sm);
   TRY_R(reset_solve_state(hb, tm));
   const unsigned grid = (unsigned)(tm.ntj * tm.ntk);
   SorArgs a{itmax, epsi, hb->omega, prof_log(), res_tol, dt, hb->sor_rev, fast};
@@ -1656,7 +1770,7 @@ int launch_sor(HostBlock* hb, int64_t itmax, double dt, double epsi, double res_
   gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
   void* args[] = {(void*)&B, (void*)&a, (void*)&gb, (void*)&tm};
   prof_mark(true);
-  BCFD_CUDA(launch_coop((const void*)k_sor64, grid, threads, args));
+  BCFD_CUDA(launch_coop(fn, grid, threads, args));
   prof_mark(false);
   BCFD_LAUNCHED();
   return launch_residual(hb, dt);
@@ -1958,17 +2072,17 @@ int launch_sor_set(const std::vector<HostBlock*>& hbs, int64_t itmax, double dt,
     for (HostBlock* hb : hbs) TRY_R(launch_sor(hb, itmax, dt, epsi, res_tol, fast));
     return 0;
   }
-  const int threads = 512;
-  for (HostBlock* hb : hbs) {
-    k_rhs<<<grid_for(hb->d.d.npacked(), 256), 256, 0, stream()>>>(hb->d, dt);
-    BCFD_LAUNCHED();
-  }
-  auto make = [&](HostBlock* hb, SorArgs& a) -> int {
-    a = SorArgs{itmax, epsi, hb->omega, prof_log(), res_tol, dt, hb->sor_rev, fast};
-    // blocks with their own launch shape keep their own launch
+  const int threads = kSor64Threads;
+  // blocks with their own launch shape keep their own launch
+  auto alone = [](const HostBlock* hb) {
     return hb->solve_threads > 0 || hb->solve_sync != 0 || hb->solve_ctas_per_sm > 0;
   };
-  // a block solved alone goes through launch_sor (which recomputes b/dt)
+  for (HostBlock* hb : hbs)
+    if (!alone(hb)) TRY_R(launch_rhs(hb, dt, fast));
+  auto make = [&](HostBlock* hb, SorArgs& a) -> int {
+    a = SorArgs{itmax, epsi, hb->omega, prof_log(), res_tol, dt, hb->sor_rev, fast};
+    return alone(hb);
+  };
   auto solo = [&](HostBlock* hb) -> int { return launch_sor(hb, itmax, dt, epsi, res_tol, fast); };
   TRY_R(launch_solve_set<SorArgs>(hbs, (const void*)k_sor64_set, threads, 0, make, solo));
   for (HostBlock* hb : hbs) TRY_R(launch_residual(hb, dt));

@@ -426,7 +426,7 @@ int bcfd_block_set_mixed_params(bcfd_handle h, int64_t inner_sweeps, double omeg
  * in the reference) */
 int bcfd_block_get_mixed_omega(bcfd_handle h, double* omega);
 /* launch shape of a block's tiled Poisson solves (the autotuner's knobs; no
- * effect on results): threads per CTA (0 = the default: 512 for the FP64
+ * effect on results): threads per CTA (0 = the default: 256 for the FP64
  * solve, 256 for the mixed one, which takes at most 256; else 128/256/512), cap
  * on co-resident CTAs per SM (0 = occupancy limit), and the FP64 solve's
  * phase sync (0 point-to-point between neighbour tiles, 1 grid-wide) */
