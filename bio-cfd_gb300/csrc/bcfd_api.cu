@@ -1366,7 +1366,7 @@ int bcfd_block_get_mixed_omega(bcfd_handle h, double* omega) {
 int bcfd_block_set_mixed_params(bcfd_handle h, int64_t inner_sweeps, double omega, int variant) {
   LOCK();
   GETB(h);
-  if (inner_sweeps < 0 || inner_sweeps > 100000 || omega < 0.0 || omega >= 2.0 || variant < 0 || variant > 5 ||
+  if (inner_sweeps < 0 || inner_sweeps > 100000 || omega < 0.0 || omega >= 2.0 || variant < 0 || variant > 6 ||
       variant == 2)  // the cluster-resident variant was withdrawn
     return BCFD_E_ARG;
   hb->dc_inner = (int)inner_sweeps;

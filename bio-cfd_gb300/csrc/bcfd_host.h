@@ -99,6 +99,7 @@ struct HostBlock {
   double lcoef_dt = 0.0;           // the deltat they were computed for (0: not computed)
   float* coef_f32 = nullptr;       // device Acx/Acy/Acz rounded to FP32
   float* pcf2 = nullptr;           // second FP32 correction buffer (both colours) of the temporal-blocked sweeps
+  unsigned long long* ll = nullptr;  // packet slots of the resident sweeps
   int64_t mk = 0, mkx1 = 0, mkx2 = 0;  // findDistnode's extreme surface nodes (1-based)
   // fine-block moves (src/Search.F90:997-1370): the last move and the index
   // ranges of the old (cpy) and new (cpy_mv) positions of the moved data,
@@ -116,7 +117,7 @@ struct HostBlock {
   int dc_inner = 0;
   double dc_omega = 0.0;
   // mixed solve kernel: 0 = library default, 1 = grid-wide phase barriers,
-  // 3 = neighbour sync, 4 = temporal-blocked
+  // 3 = neighbour sync, 4 = temporal-blocked, 5 = z-marching, 6 = resident
   int dc_variant = 0;
   int solve_threads = 0;           // threads per CTA of the tiled solves (0: 256)
   int solve_ctas_per_sm = 0;       // co-resident CTAs per SM cap (0: occupancy limit)
@@ -266,6 +267,7 @@ int launch_sor_set(const std::vector<HostBlock*>& hbs, int64_t itmax, double dt,
                    int fast = 0);
 bool tb_solve_fits(HostBlock* hb);
 bool zm_solve_fits(HostBlock* hb);
+bool res_solve_fits(HostBlock* hb);
 double mixed_omega_of(const HostBlock* hb);
 int launch_sor_mixed_set(const std::vector<HostBlock*>& hbs, int64_t itmax, double dt, double div_tol);
 // res_tol > 0: stop on the FP64 residual dt*max|b/dt - A pc| <= res_tol

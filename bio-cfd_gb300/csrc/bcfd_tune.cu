@@ -152,8 +152,9 @@ int tune_block(HostBlock* hb, Tuned* out) {
   // {256, 4, *} selects the 64-register instantiation of the FP32 solve
   // {512, 0, 4}: the temporal-blocked sweeps (small blocks)
   // {384, 0, 5}: the z-marching TMA sweeps (large blocks)
+  // {512, 0, 1}: the resident sweeps (blocks that fit the SMs' shared memory)
   static const Shape c32[] = {{128, 0, 1}, {256, 0, 1}, {128, 0, 3}, {256, 0, 3}, {256, 2, 1},
-                              {256, 1, 1}, {256, 4, 1}, {256, 4, 3}, {512, 0, 4}, {384, 0, 5}};
+                              {256, 1, 1}, {256, 4, 1}, {256, 4, 3}, {512, 0, 4}, {384, 0, 5}, {512, 0, 1}};
   Saved sv;
   if (const int e = save_state(hb, sv, false)) {
     cudaFree(sv.buf);
@@ -176,6 +177,7 @@ int tune_block(HostBlock* hb, Tuned* out) {
     if (r) break;
     if (s.sync == 4 && !tb_solve_fits(hb)) continue;
     if (s.sync == 5 && !zm_solve_fits(hb)) continue;
+    if (s.sync == 1 && s.threads == 512 && !res_solve_fits(hb)) continue;
     apply(hb, s, true);
     float ms = 0;
     if ((r = time_trial(hb, true, 16, &ms))) break;

@@ -1412,6 +1412,442 @@ __global__ void __launch_bounds__(kZmThreads, 1) k_sor_zm(DevBlock B, DcArgs a, 
   }
 }
 
+// ---------------------------------------------------------------------------
+// Resident FP32 sweeps (variant 6): one CTA per SM keeps its tile's correction
+// e, right-hand side and masks in shared memory for a whole correction, and
+// the tiles exchange edge rows once per sweep pair, without any barrier
+// between CTAs.  A pair needs the black values of the neighbours' rows within
+// two of the tile (and the four rows diagonal to its corners): the red
+// half-sweep runs over the tile and the rows next to it, the black one over
+// the tile.  The red rows next to the tile are recomputed from the inputs and
+// with the operations of the CTA that owns them, so every cell gets exactly
+// the values of the two-barrier sweep (bitwise).
+//
+// Black edge rows travel as packets {value, pair number} of 8 bytes, stored by
+// the owner and polled by the readers until the pair they need has arrived:
+// one store-to-load latency through L2 per pair, partly hidden behind the
+// tile's inner rows (edge rows go first in the black half-sweep, inner rows
+// before the poll in the red one), where the tiled solve pays two grid
+// barriers and reads e, right-hand side and masks from L2 in each half-sweep.
+// Two packet buffers alternate by pair: a tile stores pair n + 2 after it has
+// read all its neighbours' pair n + 1, which they stored after reading pair n.
+// Pair numbers count on over the corrections of a launch; the buffers are
+// zeroed before it.  At a correction's first pair every e is 0 and nothing is
+// read.
+//
+// A half-sweep's x-parity is a template parameter: one half of the CTA's warps
+// updates the rows of parity 0, the other those of parity 1, and a thread
+// keeps one run position a, so the x coefficients stay in registers over its
+// rows.
+// ---------------------------------------------------------------------------
+constexpr int kResThreads = 512;
+
+struct ResArgs {
+  int tj, tk, ntj, ntk;
+  int half;                   // threads per parity group (blockDim.x == 2 * half)
+  unsigned long long* ll[2];  // packets, one per black packed position
+};
+
+// rows of a tile in shared memory (row (jj, kk) of the tile, from (0, 0)):
+// black e from (-2, -2), red e and its right-hand side and masks from
+// (-1, -1), the black ones from (0, 0)
+struct ResTile {
+  Tile t;
+  int nq, nxh, slots;
+  float *eb, *er, *rb, *rr;
+  uint8_t *mb, *mr;
+  const float4 *ay, *az;  // y and z coefficients of rows jj >= -1 and lines kk >= -1
+  __device__ __forceinline__ int black(int jj, int kk) const { return (kk + 2) * (t.nj + 4) + jj + 2; }
+  __device__ __forceinline__ int red(int jj, int kk) const { return (kk + 1) * (t.nj + 2) + jj + 1; }
+  __device__ __forceinline__ int own(int jj, int kk) const { return kk * t.nj + jj; }
+};
+
+// A half-sweep's work is cut into segments: rows jj, jj + 2, ... of one line kk
+// (one x-parity), stored as kk + 2 | jj + 2 << 8 | rows << 16.  Lists per
+// parity of j + k: the red rows whose black neighbours all lie in the tile, the
+// other red rows, the black lines next to the tile's k faces, the other black
+// lines; then the halo rows (kk + 2 | jj + 2 << 8).
+enum ResList { RL_RED_IN = 0, RL_RED_OUT = 2, RL_BLACK = 4, RL_BLACK_LATE = 5, RL_HALO = 8, RL_COUNT = 9 };
+
+__device__ __forceinline__ ulonglong2 ld_packets(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_packets(ulonglong2* p, unsigned long long a, unsigned long long b) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void write_run(unsigned long long* slot, unsigned pair, const float4& v) {
+  ulonglong2* p = reinterpret_cast<ulonglong2*>(slot);
+  const unsigned long long hi = (unsigned long long)pair << 32;
+  st_packets(p, hi | __float_as_uint(v.x), hi | __float_as_uint(v.y));
+  st_packets(p + 1, hi | __float_as_uint(v.z), hi | __float_as_uint(v.w));
+}
+
+// what a thread keeps over its rows: the run's x coefficients, and the
+// reciprocals of the diagonal for the y and z diagonal terms ly, lz
+struct ResCoef {
+  float a1[4], a2[4], a3[4], ri[4], ly, lz;
+};
+
+// one half-sweep of colour C over this thread's share (every R.slots-th
+// segment from `slot`) of a segment list, x-parity PAR: tile_half32's
+// operations, its division by the diagonal as the product
+// with the diagonal's reciprocal (__fdividef(s, d) and s * __fdividef(1, d)
+// are the same bits for every normal d), which is kept while the row's y and z
+// diagonal terms repeat (on a uniform grid it is formed once).  Black rows
+// within two of the tile's faces are stored as packets of `pair` too.
+template <int C, int PAR>
+__device__ __forceinline__ void res_segments(const DevBlock& B, const ResTile& R, const unsigned* list, int n, int a,
+                                             int slot, ResCoef& K, unsigned long long* ll, unsigned pair,
+                                             float omega) {
+  const int nxh = R.nxh, nj = R.t.nj, nk = R.t.nk;
+  const int sk = (C ? nj + 4 : nj + 2) * nxh;  // one line of the other colour
+  for (int q = slot; q < n; q += R.slots) {
+    const unsigned seg = list[q];
+    const int kk = (int)(seg & 255u) - 2, j0 = (int)((seg >> 8) & 255u) - 2, rows = (int)(seg >> 16);
+    const float* __restrict__ o = (C ? R.eb + R.black(j0, kk) * nxh : R.er + R.red(j0, kk) * nxh) + 4 * a;
+    float* __restrict__ own = (C ? R.er + R.red(j0, kk) * nxh : R.eb + R.black(j0, kk) * nxh) + 4 * a;
+    const int rw = C ? R.red(j0, kk) : R.own(j0, kk);
+    const float* __restrict__ rhs = (C ? R.rr : R.rb) + rw * nxh + 4 * a;
+    const uint8_t* __restrict__ mk = (C ? R.mr : R.mb) + rw * R.nq + a;
+    const float4* __restrict__ ay = R.ay + j0 + 1;
+    const float4 cz = R.az[kk + 1];
+    float4 os = *reinterpret_cast<const float4*>(o - nxh);
+    const int edge = C == 0 && (kk < 2 || kk >= nk - 2);
+    unsigned long long* slot_ll =
+        C ? nullptr : ll + (int64_t)nxh * ((R.t.j0 + j0 - 1) + (int64_t)B.d.NY * (R.t.k0 + kk - 1)) + 4 * a;
+    for (int u = 0; u < rows; ++u) {
+      const float4 oc = *reinterpret_cast<const float4*>(o), on = *reinterpret_cast<const float4*>(o + nxh);
+      const float4 ob = *reinterpret_cast<const float4*>(o - sk), ot = *reinterpret_cast<const float4*>(o + sk);
+      const float ox = PAR ? o[4] : o[-1];
+      const float4 r4 = *reinterpret_cast<const float4*>(rhs), e4 = *reinterpret_cast<const float4*>(own);
+      const float4 cy = *ay;
+      const unsigned m = *mk;
+      if (cy.y != K.ly || cz.y != K.lz) {
+        K.ly = cy.y;
+        K.lz = cz.y;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) K.ri[c] = __fdividef(1.0f, K.a2[c] + cy.y + cz.y);
+      }
+      const float oxs[5] = {PAR ? oc.x : ox, PAR ? oc.y : oc.x, PAR ? oc.z : oc.y, PAR ? oc.w : oc.z, PAR ? ox : oc.w};
+      const float sv[4] = {os.x, os.y, os.z, os.w}, nv[4] = {on.x, on.y, on.z, on.w};
+      const float bv[4] = {ob.x, ob.y, ob.z, ob.w}, tv[4] = {ot.x, ot.y, ot.z, ot.w};
+      const float rv[4] = {r4.x, r4.y, r4.z, r4.w}, ev[4] = {e4.x, e4.y, e4.z, e4.w};
+      float v[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float s = rv[c];
+        s = __fmaf_rn(-K.a1[c], oxs[c], s);
+        s = __fmaf_rn(-K.a3[c], oxs[c + 1], s);
+        s = __fmaf_rn(-cy.x, sv[c], s);
+        s = __fmaf_rn(-cy.z, nv[c], s);
+        s = __fmaf_rn(-cz.x, bv[c], s);
+        s = __fmaf_rn(-cz.z, tv[c], s);
+        v[c] = __fmaf_rn(omega, s * K.ri[c] - ev[c], ev[c]);
+      }
+      if (m != 15u) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = (m >> c) & 1u ? v[c] : ev[c];
+      }
+      const float4 v4 = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4*>(own) = v4;
+      if (C == 0) {
+        const int jj = j0 + 2 * u;
+        if (edge || jj < 2 || jj >= nj - 2) write_run(slot_ll, pair, v4);
+        slot_ll += 2 * nxh;
+      }
+      os = on;
+      o += 2 * nxh;
+      own += 2 * nxh;
+      rhs += 2 * nxh;
+      ay += 2;
+      mk += 2 * R.nq;
+    }
+  }
+}
+
+// the halo rows of pair `pair` into shared memory; all of a thread's first
+// four runs' loads are in flight together.  false: the wait gave up
+__device__ __forceinline__ bool res_import(const DevBlock& B, const ResTile& R, const unsigned* list, int n,
+                                           const unsigned long long* ll, unsigned pair, const GridBar& gb) {
+  constexpr int U = 2;
+  const int total = n * R.nq, nxh = R.nxh;
+  unsigned long long t0 = 0;
+  unsigned spins = 0;
+  for (int q0 = threadIdx.x; q0 < total; q0 += U * blockDim.x) {
+    const ulonglong2* p[U];
+    float4* dst[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * blockDim.x;
+      p[u] = nullptr;
+      if (q < total) {
+        const int row = q / R.nq, a = q - row * R.nq;
+        const int kk = (int)(list[row] & 255u) - 2, jj = (int)(list[row] >> 8) - 2;
+        const int j = R.t.j0 + jj, k = R.t.k0 + kk;
+        p[u] = reinterpret_cast<const ulonglong2*>(ll + (int64_t)nxh * ((j - 1) + (int64_t)B.d.NY * (k - 1)) + 4 * a);
+        dst[u] = reinterpret_cast<float4*>(R.eb + R.black(jj, kk) * nxh + 4 * a);
+      }
+    }
+    for (;;) {
+      ulonglong2 x[U], y[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (p[u]) {
+          x[u] = ld_packets(p[u]);
+          y[u] = ld_packets(p[u] + 1);
+        }
+      bool more = false;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (p[u]) {
+          if ((unsigned)(x[u].x >> 32) == pair && (unsigned)(x[u].y >> 32) == pair &&
+              (unsigned)(y[u].x >> 32) == pair && (unsigned)(y[u].y >> 32) == pair) {
+            *dst[u] = make_float4(__uint_as_float((unsigned)x[u].x), __uint_as_float((unsigned)x[u].y),
+                                  __uint_as_float((unsigned)y[u].x), __uint_as_float((unsigned)y[u].y));
+            p[u] = nullptr;
+          } else {
+            more = true;
+          }
+        }
+      if (!more) break;
+      if ((++spins & 63u) == 0) {
+        if (t0 == 0) t0 = globaltimer_ns();
+        if ((ld_relaxed_u64(gb.ctr) & kBarAbandon) || ld_acquire_i(gb.err) != 0) return false;
+        if (globaltimer_ns() - t0 > gb.limit_ns) {
+          atomicCAS(gb.err, 0, BCFD_E_TIMEOUT);
+          return false;
+        }
+      }
+    }
+  }
+  return true;
+}
+
+// shared memory of a tile: four guard floats before each e array and after the
+// last, the right-hand sides, the y and z coefficients, the masks and the lists
+// (at most one segment per row of a colour)
+struct ResLayout {
+  int nb, nr, no;  // rows of black e, of red e, of the tile
+  size_t coef, mask, list, bytes;
+};
+__host__ __device__ inline ResLayout res_layout(int nxh, int nj, int nk) {
+  ResLayout L;
+  L.nb = (nj + 4) * (nk + 4);
+  L.nr = (nj + 2) * (nk + 2);
+  L.no = nj * nk;
+  L.coef = ((size_t)(L.nb + 2 * L.nr + L.no) * nxh + 12) * sizeof(float);
+  L.mask = L.coef + (size_t)(nj + nk + 4) * sizeof(float4);
+  L.list = L.mask + (((size_t)(L.nr + L.no) * (nxh / 4) + 15) & ~(size_t)15);
+  L.bytes = L.list + (size_t)(L.nr + L.no + 4 * (nj + nk) + 4) * sizeof(unsigned);
+  return L;
+}
+
+// x += e in FP64 over the tile's updated cells of colour C
+template <int C>
+__device__ __forceinline__ void res_apply(const DevBlock& B, const ResTile& R) {
+  const Dims& d = B.d;
+  double* __restrict__ x = B.pc[C];
+  const int64_t sz = (int64_t)d.NXH * d.NY;
+  const int n = R.nq * R.t.nj * R.t.nk;
+  Walk3 w;
+  w.init(threadIdx.x, blockDim.x, R.nq, R.t.nj);
+  for (int q = threadIdx.x; q < n; q += blockDim.x, w.next()) {
+    const int64_t pi = (int64_t)d.NXH * (R.t.j0 + w.b - 1) + sz * (R.t.k0 + w.c - 1) + 4 * w.a;
+    const unsigned m = C ? R.mr[R.red(w.b, w.c) * R.nq + w.a] : R.mb[R.own(w.b, w.c) * R.nq + w.a];
+    const float4 e4 = *reinterpret_cast<const float4*>(
+        (C ? R.er + R.red(w.b, w.c) * R.nxh : R.eb + R.black(w.b, w.c) * R.nxh) + 4 * w.a);
+    double2 a = *reinterpret_cast<const double2*>(x + pi);
+    double2 b = *reinterpret_cast<const double2*>(x + pi + 2);
+    if (m & 1u) a.x = a.x + (double)e4.x;
+    if (m & 2u) a.y = a.y + (double)e4.y;
+    if (m & 4u) b.x = b.x + (double)e4.z;
+    if (m & 8u) b.y = b.y + (double)e4.w;
+    *reinterpret_cast<double2*>(x + pi) = a;
+    *reinterpret_cast<double2*>(x + pi + 2) = b;
+  }
+}
+
+__global__ void __launch_bounds__(kResThreads, 1) k_sor_res(DevBlock B, DcArgs a, GridBar gb, ResArgs z) {
+  extern __shared__ float4 res_raw[];
+  __shared__ double sh[32];
+  __shared__ int cnt[RL_COUNT], off[RL_COUNT];
+  const Dims& d = B.d;
+  const int cta = (int)blockIdx.x;
+  ResTile R;
+  R.t = my_tile(d, TileMap{z.tj, z.tk, z.ntj, z.ntk, nullptr, 1}, cta);
+  R.nxh = d.NXH;
+  R.nq = d.NXH >> 2;
+  const int nj = R.t.nj, nk = R.t.nk, nq = R.nq;
+  const ResLayout L = res_layout(d.NXH, nj, nk);
+  float* f = reinterpret_cast<float*>(res_raw);
+  R.eb = f + 4;
+  R.er = R.eb + L.nb * R.nxh + 4;
+  R.rr = R.er + L.nr * R.nxh + 4;
+  R.rb = R.rr + L.nr * R.nxh;
+  char* const raw = reinterpret_cast<char*>(res_raw);
+  float4* const coef = reinterpret_cast<float4*>(raw + L.coef);
+  R.ay = coef;
+  R.az = coef + nj + 2;
+  R.mr = reinterpret_cast<uint8_t*>(raw + L.mask);
+  R.mb = R.mr + L.nr * nq;
+  unsigned* const lists = reinterpret_cast<unsigned*>(raw + L.list);
+  R.slots = z.half / nq;
+  for (int q = threadIdx.x; q < nj + nk + 4; q += blockDim.x) {
+    const int row = q < nj + 2 ? R.t.j0 + q - 1 : R.t.k0 + (q - nj - 2) - 1, n = q < nj + 2 ? d.ny : d.nz;
+    if (row >= 2 && row <= n + 1) coef[q] = q < nj + 2 ? B.ayr[row - 2] : B.azr[row - 2];
+  }
+  // rows per segment: about what a slot has to do per half-sweep
+  const int len_r = max(1, (L.nr / 2 + R.slots - 1) / R.slots), len_b = max(1, (L.no / 2 + R.slots - 1) / R.slots);
+  // the segments of rows lo .. hi of line kk at parity p of j + k
+  auto cut = [&](int list, int kk, int lo, int hi, int p, int len, auto&& put) {
+    for (int jj = lo + ((R.t.j0 + lo + R.t.k0 + kk + p) & 1); jj <= hi; jj += 2 * len)
+      put(list, (unsigned)(kk + 2) | (unsigned)(jj + 2) << 8 | (unsigned)(min(len, (hi - jj) / 2 + 1)) << 16);
+  };
+  const int lo = R.t.j0 > 2 ? -1 : 0, hi = R.t.j0 + nj <= d.ny + 1 ? nj : nj - 1;  // red rows of an inner line
+  auto each_line = [&](auto&& put) {
+    for (int q = threadIdx.x; q < 2 * (nk + 4); q += blockDim.x) {
+      const int kk = q / 2 - 2, p = q & 1, k = R.t.k0 + kk;
+      if (k < 2 || k > d.nz + 1) continue;  // ghost lines: e stays 0
+      const int ok = kk < 0 ? -kk : kk >= nk ? kk - nk + 1 : 0;
+      // halo rows within two of the tile, and diagonal to its corners
+      if (p == 0)
+        for (int jj = -2; jj < nj + 2; ++jj) {
+          const int j = R.t.j0 + jj, oj = jj < 0 ? -jj : jj >= nj ? jj - nj + 1 : 0;
+          if (j >= 2 && j <= d.ny + 1 && oj + ok > 0 && oj + ok <= 2)
+            put((int)RL_HALO, (unsigned)(kk + 2) | (unsigned)(jj + 2) << 8);
+        }
+      if (ok > 1) continue;
+      if (ok == 1) {
+        cut(RL_RED_OUT + p, kk, 0, nj - 1, p, len_r, put);
+        continue;
+      }
+      if (kk == 0 || kk == nk - 1 || nj <= 2) {
+        cut(RL_RED_OUT + p, kk, lo, hi, p, len_r, put);
+      } else {
+        cut(RL_RED_IN + p, kk, 1, nj - 2, p, len_r, put);
+        cut(RL_RED_OUT + p, kk, lo, 0, p, len_r, put);
+        cut(RL_RED_OUT + p, kk, nj - 1, hi, p, len_r, put);
+      }
+      cut((kk < 2 || kk >= nk - 2 ? RL_BLACK : RL_BLACK_LATE) + 2 * p, kk, 0, nj - 1, p, len_b, put);
+    }
+  };
+  if (threadIdx.x < RL_COUNT) cnt[threadIdx.x] = 0;
+  __syncthreads();
+  each_line([&](int l, unsigned) { atomicAdd(&cnt[l], 1); });
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int at = 0;
+    for (int l = 0; l < RL_COUNT; ++l) {
+      off[l] = at;
+      at += cnt[l];
+      cnt[l] = 0;
+    }
+  }
+  __syncthreads();
+  each_line([&](int l, unsigned v) { lists[off[l] + atomicAdd(&cnt[l], 1)] = v; });
+  // the run masks of red rows next to the tile and of the tile's rows
+  const int64_t sz = (int64_t)d.NXH * d.NY;
+  auto mask4 = [&](int c, int64_t pi) {
+    const uchar4 m = *reinterpret_cast<const uchar4*>(B.upd[c] + pi);
+    return (uint8_t)((m.x != 0) | ((m.y != 0) << 1) | ((m.z != 0) << 2) | ((m.w != 0) << 3));
+  };
+  for (int q = threadIdx.x; q < L.nr * nq; q += blockDim.x) {
+    const int row = q / nq, ra = q - row * nq;
+    const int jj = row % (nj + 2) - 1, kk = row / (nj + 2) - 1;
+    // rows jj = -1 .. nj and kk = -1 .. nk lie inside the arrays (ghost rows
+    // hold no updated cell)
+    const int64_t pi = (int64_t)d.NXH * (R.t.j0 + jj - 1) + sz * (R.t.k0 + kk - 1) + 4 * ra;
+    R.mr[q] = mask4(1, pi);
+    if (jj >= 0 && jj < nj && kk >= 0 && kk < nk) R.mb[R.own(jj, kk) * nq + ra] = mask4(0, pi);
+  }
+  // this thread's parity group, run position and first row
+  const bool odd = (int)threadIdx.x >= z.half;
+  const int lt = (int)threadIdx.x - (odd ? z.half : 0);
+  const int pa = lt % nq, slot = lt / nq < R.slots ? lt / nq : 0x40000000;
+  ResCoef K;
+  {
+    const float4* ar = B.axr + 3 * (odd ? 1 : 0) * nq + pa;
+    const float4 c1 = ar[0], c2 = ar[nq], c3 = ar[2 * nq];
+    const float f1[4] = {c1.x, c1.y, c1.z, c1.w}, f2[4] = {c2.x, c2.y, c2.z, c2.w}, f3[4] = {c3.x, c3.y, c3.z, c3.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      K.a1[c] = f1[c];
+      K.a2[c] = f2[c];
+      K.a3[c] = f3[c];
+      K.ri[c] = 0.f;
+    }
+    K.ly = K.lz = __int_as_float(0x7fc00000);  // NaN: no reciprocals yet
+  }
+  BlockStats* st = B.stats;
+  int64_t sweeps = 0;
+  double res = 0.0, res_prev = 0.0;
+  int inner = a.inner;
+  unsigned pair = 0;
+  int outer = 0;
+  for (;; ++outer) {
+    double m = nmax(tile_residual64v<1>(B, R.t, a.inv_dt), tile_residual64v<0>(B, R.t, a.inv_dt));
+    m = block_max(m, sh);
+    if (threadIdx.x == 0) atomic_max_nonneg(&st->slot[outer % 3], m);
+    if (!grid_sync(gb)) return;
+    res = take_slot(st, outer, cta);
+    if (a.dt * res <= a.div_tol || outer >= a.max_outer || non_finite(res)) break;
+    inner = next_inner(a, outer, res, res_prev, inner);
+    res_prev = res;
+    // e = 0 and the right-hand sides (the rows next to the tile come from
+    // their owners' residual pass: read through L2)
+    for (int q = threadIdx.x; q < ((L.nb + L.nr) * R.nxh + 12) / 4; q += blockDim.x)
+      res_raw[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = threadIdx.x; q < L.nr * nq; q += blockDim.x) {
+      const int row = q / nq, ra = q - row * nq;
+      const int jj = row % (nj + 2) - 1, kk = row / (nj + 2) - 1;
+      const int64_t pi = (int64_t)d.NXH * (R.t.j0 + jj - 1) + sz * (R.t.k0 + kk - 1) + 4 * ra;
+      *reinterpret_cast<float4*>(R.rr + 4 * q) = __ldcg(reinterpret_cast<const float4*>(B.rhsf[1] + pi));
+      if (jj >= 0 && jj < nj && kk >= 0 && kk < nk)
+        *reinterpret_cast<float4*>(R.rb + R.own(jj, kk) * R.nxh + 4 * ra) =
+            __ldcg(reinterpret_cast<const float4*>(B.rhsf[0] + pi));
+    }
+    __syncthreads();
+    // rows of the group: red of x-parity PAR sit at j + k of parity PAR,
+    // black at the other
+    const int pr = odd ? 1 : 0, pb = 1 - pr;
+    for (int it = 0; it < inner; ++it) {
+      const unsigned long long* rl = z.ll[pair & 1];
+      ++pair;
+      unsigned long long* wl = z.ll[pair & 1];
+      bool ok = true;
+      auto red = [&](int l) {
+        if (odd) res_segments<1, 1>(B, R, lists + off[l], cnt[l], pa, slot, K, nullptr, 0, a.omega);
+        else res_segments<1, 0>(B, R, lists + off[l], cnt[l], pa, slot, K, nullptr, 0, a.omega);
+      };
+      red(RL_RED_IN + pr);
+      if (it > 0) ok = res_import(B, R, lists + off[RL_HALO], cnt[RL_HALO], rl, pair - 1, gb);
+      if (__syncthreads_or(!ok)) {
+        if (threadIdx.x == 0) atomicOr(gb.ctr, kBarAbandon);
+        return;
+      }
+      red(RL_RED_OUT + pr);
+      __syncthreads();
+      const int l = RL_BLACK + 2 * pb, nbk = cnt[l] + cnt[l + 1];
+      if (odd) res_segments<0, 1>(B, R, lists + off[l], nbk, pa, slot, K, wl, pair, a.omega);
+      else res_segments<0, 0>(B, R, lists + off[l], nbk, pa, slot, K, wl, pair, a.omega);
+      __syncthreads();
+    }
+    sweeps += inner;
+    res_apply<1>(B, R);
+    res_apply<0>(B, R);
+    if (!grid_sync(gb)) return;
+  }
+  if (cta == 0 && threadIdx.x == 0) {
+    log_solve(a.log, sweeps, outer + 1, B.cnt[C_FLUID], 1);
+    st->niter = st->niter + sweeps;
+    st->derr2 = a.dt * res;
+    st->pad[1] = a.dt * res;
+    if (non_finite(res)) set_err(B.err, BCFD_E_NONFINITE);
+  }
+}
+
 // Several blocks' solves in one cooperative launch: member m owns CTAs
 // [cta0, cta0 + its tile count) and has its own barrier, tiles and slots.
 constexpr int kMaxSolveBatch = 16;
@@ -1821,6 +2257,18 @@ bool tb_solve_fits(HostBlock* hb) {
   return tb_tiles(hb, &a, &b) != 0;
 }
 
+static DcArgs mixed_args(const HostBlock* hb, int64_t itmax, double dt, double div_tol) {
+  DcArgs a;
+  a.inner = hb->dc_inner > 0 ? hb->dc_inner : 64;
+  a.omega = (float)mixed_omega_of(hb);
+  a.max_outer = itmax / a.inner + 1;
+  a.dt = dt;
+  a.inv_dt = 1.0 / dt;
+  a.div_tol = div_tol;
+  a.log = prof_log();
+  return a;
+}
+
 static int launch_sor_tb(HostBlock* hb, int64_t itmax, double dt, double div_tol) {
   DevBlock& B = hb->d;
   TRY_R(ensure_second_buffer(hb));
@@ -1831,15 +2279,7 @@ static int launch_sor_tb(HostBlock* hb, int64_t itmax, double dt, double div_tol
   const size_t smem = tb_bytes(B.d, tj, tk);
   BCFD_CUDA(cudaFuncSetAttribute((const void*)k_sor_tb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const unsigned grid = (unsigned)(tm.ntj * tm.ntk);
-  DcArgs a;
-  a.inner = hb->dc_inner > 0 ? hb->dc_inner : 64;
-  double om = hb->dc_omega > 0 ? hb->dc_omega : mixed_omega_default(B.d);
-  a.omega = (float)std::min(kMixedOmegaMax, std::max(1.0, om));
-  a.max_outer = itmax / a.inner + 1;
-  a.dt = dt;
-  a.inv_dt = 1.0 / dt;
-  a.div_tol = div_tol;
-  a.log = prof_log();
+  DcArgs a = mixed_args(hb, itmax, dt, div_tol);
   GridBar gb = make_bar(B.err, grid);
   gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
   float* e2 = hb->pcf2;
@@ -1955,15 +2395,7 @@ static int launch_sor_zm(HostBlock* hb, int64_t itmax, double dt, double div_tol
   const size_t smem = zm_smem_bytes(B.d, z.rows);
   BCFD_CUDA(cudaFuncSetAttribute((const void*)k_sor_zm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const unsigned grid = (unsigned)(z.ntj * z.nzs);
-  DcArgs a;
-  a.inner = hb->dc_inner > 0 ? hb->dc_inner : 64;
-  double om = hb->dc_omega > 0 ? hb->dc_omega : mixed_omega_default(B.d);
-  a.omega = (float)std::min(kMixedOmegaMax, std::max(1.0, om));
-  a.max_outer = itmax / a.inner + 1;
-  a.dt = dt;
-  a.inv_dt = 1.0 / dt;
-  a.div_tol = div_tol;
-  a.log = prof_log();
+  DcArgs a = mixed_args(hb, itmax, dt, div_tol);
   GridBar gb = make_bar(B.err, grid);
   gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
   void* args[] = {(void*)&B, (void*)&a, (void*)&gb, (void*)&z, (void*)&maps};
@@ -1974,9 +2406,94 @@ static int launch_sor_zm(HostBlock* hb, int64_t itmax, double dt, double div_tol
   return 0;
 }
 
+// Resident solve (variant 6): the tile that gives the fullest SM the fewest
+// rows (one CTA per SM), squarest among equals; 0 when it does not fit in
+// shared memory.
+static int res_shape(HostBlock* hb, ResArgs* z, size_t* bytes) {
+  const Dims& d = hb->d.d;
+  const int nq = d.NXH / 4;
+  if (nq > kResThreads / 2) return 0;
+  int smem_max = 0;
+  if (cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, lib().device) != cudaSuccess)
+    return 0;
+  const size_t cap = (size_t)smem_max - 1024;  // static shared memory of the kernel
+  const int nsm = num_sms();
+  long best = -1;
+  int per = 0;
+  for (int ntj = 1; ntj <= std::min(d.ny, nsm); ++ntj) {
+    const int tj = (d.ny + ntj - 1) / ntj;
+    if ((d.ny + tj - 1) / tj != ntj || tj > 250) continue;
+    const int ntk0 = std::min(d.nz, nsm / ntj);
+    const int tk = (d.nz + ntk0 - 1) / ntk0, ntk = (d.nz + tk - 1) / tk;
+    if (tk > 250) continue;
+    // the red half-sweep's rows, the rows next to the tile among them
+    const long rows = (long)(tj + 2) * (tk + 2) + (long)tj * tk;
+    if (best < 0 || rows < best || (rows == best && tj + tk < per)) {
+      best = rows;
+      per = tj + tk;
+      z->tj = tj;
+      z->ntj = ntj;
+      z->tk = tk;
+      z->ntk = ntk;
+    }
+  }
+  if (best < 0) return 0;
+  *bytes = res_layout(d.NXH, z->tj, z->tk).bytes;
+  if (*bytes > cap) return 0;
+  // threads per parity group: whole lines of runs, as many as the rows can
+  // use, padded to warps
+  const int lines = std::max(1, std::min(kResThreads / 2 / nq, ((z->tj + 2) * (z->tk + 2) + 1) / 2));
+  z->half = std::min(kResThreads / 2, (lines * nq + 31) / 32 * 32);
+  return 1;
+}
+
+bool res_solve_fits(HostBlock* hb) {
+  ResArgs z{};
+  size_t bytes = 0;
+  return res_shape(hb, &z, &bytes) != 0;
+}
+
+static int launch_sor_res(HostBlock* hb, int64_t itmax, double dt, double div_tol) {
+  DevBlock& B = hb->d;
+  ResArgs z{};
+  size_t smem = 0;
+  if (!res_shape(hb, &z, &smem)) return BCFD_E_STATE;
+  const size_t np = (size_t)B.d.npacked(), llb = 2 * np * sizeof(unsigned long long);
+  if (!hb->ll) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, llb) != cudaSuccess) return BCFD_E_NOMEM;
+    hb->allocs.push_back(p);
+    hb->ll = static_cast<unsigned long long*>(p);
+    lib().gen++;
+  }
+  BCFD_CUDA(cudaMemsetAsync(hb->ll, 0, llb, stream()));
+  z.ll[0] = hb->ll;
+  z.ll[1] = hb->ll + np;
+  TRY_R(reset_solve_state(hb, TileMap{z.tj, z.tk, z.ntj, z.ntk, hb->prog, 1}));
+  BCFD_CUDA(cudaFuncSetAttribute((const void*)k_sor_res, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DcArgs a = mixed_args(hb, itmax, dt, div_tol);
+  const unsigned grid = (unsigned)(z.ntj * z.ntk);
+  GridBar gb = make_bar(B.err, grid);
+  gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
+  void* args[] = {(void*)&B, (void*)&a, (void*)&gb, (void*)&z};
+  prof_mark(true);
+  BCFD_CUDA(launch_coop((const void*)k_sor_res, grid, (unsigned)(2 * z.half), args, smem));
+  prof_mark(false);
+  BCFD_LAUNCHED();
+  return 0;
+}
+
 int launch_sor_mixed(HostBlock* hb, int64_t itmax, double dt, double div_tol) {
   DevBlock& B = hb->d;
   const int64_t np = B.d.npacked();
+  // the resident sweeps by choice, or by default (no launch shape asked for)
+  // wherever they fit: on every such size measured they are faster than the
+  // tiled ones, 4.64 -> 1.47 us per sweep pair on 33x21x27, 5.2 -> 2.4 on 64^3,
+  // 8.2 -> 5.0 on 128x96x96, 10.3 -> 6.7 on 128^3
+  // (the autotuner names them variant 1 with kResThreads threads)
+  const bool shaped = hb->dc_variant != 0 || hb->dc_threads > 0 || hb->dc_ctas_per_sm > 0;
+  if ((hb->dc_variant == 6 || !shaped || (hb->dc_variant == 1 && hb->dc_threads == kResThreads)) && res_solve_fits(hb))
+    return launch_sor_res(hb, itmax, dt, div_tol);
   for (int c = 0; c < 2; ++c) BCFD_CUDA(cudaMemsetAsync(B.pcf[c], 0, np * sizeof(float), stream()));
   if (hb->dc_variant == 4 && tb_solve_fits(hb)) return launch_sor_tb(hb, itmax, dt, div_tol);
   if (hb->dc_variant == 5 && zm_solve_fits(hb)) return launch_sor_zm(hb, itmax, dt, div_tol);
@@ -1987,15 +2504,7 @@ int launch_sor_mixed(HostBlock* hb, int64_t itmax, double dt, double div_tol) {
   TileMap tm = choose_tiles(hb, fn, threads, hb->dc_variant == 3 ? 0 : 1, hb->dc_ctas_per_sm);
   TRY_R(reset_solve_state(hb, tm));
   const unsigned grid = (unsigned)(tm.ntj * tm.ntk);
-  DcArgs a;
-  a.inner = hb->dc_inner > 0 ? hb->dc_inner : 64;
-  double om = hb->dc_omega > 0 ? hb->dc_omega : mixed_omega_default(B.d);
-  a.omega = (float)std::min(kMixedOmegaMax, std::max(1.0, om));
-  a.max_outer = itmax / a.inner + 1;
-  a.dt = dt;
-  a.inv_dt = 1.0 / dt;
-  a.div_tol = div_tol;
-  a.log = prof_log();
+  DcArgs a = mixed_args(hb, itmax, dt, div_tol);
   GridBar gb = make_bar(B.err, grid);
   gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
   void* args[] = {(void*)&B, (void*)&a, (void*)&gb, (void*)&tm};

@@ -417,8 +417,11 @@ int bcfd_block_get_divergence(bcfd_handle h, double* out);
  * temporal-blocked sweeps, one grid barrier per sweep pair, when the block's
  * halo'd tiles fit in shared memory, else 1; 5: z-marching sweeps, two
  * sweep pairs per pass over the block with the correction staged in shared
- * memory by TMA, when a packed row fits one TMA box (nx <= 509), else 1;
- * 1, 3, 4 and 5 give bitwise the same corrections; 2 is not accepted) */
+ * memory by TMA, when a packed row fits one TMA box (nx <= 509), else 1; 6:
+ * resident sweeps, each SM keeping a tile of the correction in shared memory,
+ * when the block fits the SMs' shared memory, else 1; all of them give bitwise
+ * the same corrections; 2 is not accepted).  The library's choice is 6 where
+ * it fits, else 1 */
 int bcfd_block_set_mixed_params(bcfd_handle h, int64_t inner_sweeps, double omega, int variant);
 /* the relaxation factor block h's FP32 correction sweeps use (its setting or
  * the default: 2 / (1 + sqrt(1 - rho^2)), rho = (cos(pi/nx) + cos(pi/ny) +
@@ -432,7 +435,8 @@ int bcfd_block_get_mixed_omega(bcfd_handle h, double* omega);
  * phase sync (0 point-to-point between neighbour tiles, 1 grid-wide) */
 int bcfd_block_set_solve_launch(bcfd_handle h, int threads, int ctas_per_sm, int fp64_sync);
 /* out[6] = FP64 solve threads, CTAs/SM cap, sync; FP32 correction threads,
- * CTAs/SM cap, variant (0 = library default) */
+ * CTAs/SM cap, variant (0 = library default; 1 with 512 threads: the resident
+ * sweeps) */
 int bcfd_block_get_solve_launch(bcfd_handle h, int* out);
 /* Autotuner (no counterpart in the reference): for every block, times short
  * solves under each candidate launch shape of the FP64 solve and of the FP32
