@@ -303,6 +303,7 @@ void phase_mark(int ph);
 int launch_sor_mixed(HostBlock* hb, int64_t itmax, double dt, double div_tol);
 // k_momentum.cu
 int launch_momentum(HostBlock* hb, double dt, double re, bool fp32);
+int launch_momentum_tables(HostBlock* hb);
 int launch_momentum_tangent(HostBlock* hb, double dt, double re, const double* const du[4], double* const val[3],
                             double* const tan[3]);
 int solve_zero_bc_dev(HostBlock* hb, const double* r, double* x, double tol, int64_t itmax, bool transpose);

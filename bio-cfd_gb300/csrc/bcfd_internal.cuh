@@ -109,8 +109,15 @@ struct DevBlock {
   // FP32 copies of dxa/dya/dza and ca/ck (FP32 momentum stencil)
   const float *dxf, *dyf, *dzf;
   const float *caf[N_TAB], *ckf[N_TAB];
+  // the momentum stencil's divisors, reciprocals and grid quotients per grid
+  // line (k_momentum.cu: axes x, y, z one after the other, each slot an array
+  // over the axis), in FP64 and FP32, and a word per line on the reciprocals
+  const double* mt;
+  const float* mtf;
+  const unsigned* mtk;
   // fields
   double *u, *v, *w, *p, *ut, *vt, *wt;
+  float* mf[4];  // u, v, w, p rounded to FP32 (the FP32 momentum stencil's input)
   // tags
   int8_t *cell, *cell_n, *cell2, *nodeTag, *cell_pr;
   uint8_t* tsnear;  // 1 where a cell is within [-3,3]^3 of a TS cell (overlay stencil)

@@ -19,9 +19,71 @@ namespace bcfd {
 
 namespace {
 
+// deltat, re, and what div_any needs to divide by re (re_k: DivKind bits)
 struct MomArgs {
-  double dt, re;
+  double dt, re, re_y;
+  unsigned re_k;
 };
+
+// Divisors of the stencil along one axis at grid index q (dl, d, dr the
+// spacings of q - 1, q, q + 1; CA / CK the sixth column of the axis's own (self)
+// and transverse (cross) coefficient tables), then its grid-only quotients and
+// the tables' first five columns.  Groups of 32 indices hold 32 consecutive
+// entries per slot: a warp's x entries are contiguous and every slot sits at a
+// constant offset from a thread's first one (immediate addresses).
+enum MomDiv {
+  MD_HALF_R = 0,  // 0.5 (d + dr)
+  MD_HALF_L,      // 0.5 (d + dl)
+  MD_SA,          // CAself dr
+  MD_SK,          // (2 CKself) d
+  MD_XA,          // CAcross (0.5 (d + dr))
+  MD_XK,          // (2 CKcross) (0.5 (d + dl))
+  MD_D,           // d
+  MD_R,           // dr
+  N_MD
+};
+enum MomQuot { MQ_R = 0, MQ_2, MQ_C, N_MQ };  // dr / (d + dr), 2 / (d + dr), 2 / (0.5 ((d + dr) + (d + dl)))
+// FP64 slots: divisor and reciprocal of each MomDiv, the quotients, CA and CK
+// 1..5 self, CA and CK 1..5 cross; FP32 slots: reciprocals, quotients by
+// __fdividef, divisors, IEEE quotients, the same coefficients
+constexpr int kMtQ = 2 * N_MD, kMtC = kMtQ + N_MQ, kMtSlots = kMtC + 20;
+constexpr int kMfQ = N_MD, kMfD = kMfQ + N_MQ, kMfI = kMfD + N_MD, kMfC = kMfI + N_MQ, kMfSlots = kMfC + 20;
+
+// first entry of grid index q (0-based) of an axis whose groups start at g0
+__host__ __device__ inline int64_t mom_slot0(int g0, int q, int slots) {
+  return ((int64_t)(g0 + (q >> 5)) * slots) * 32 + (q & 31);
+}
+__host__ __device__ inline int mom_groups(int n) { return (n + 31) >> 5; }
+
+// how a divisor's reciprocal may be used: bit s of the axis word, the quotient
+// needs a second correction; bit 8 + s, the division itself is needed
+__host__ __device__ inline unsigned div_kind(double d, double y) {
+  const double m = d < 0 ? -d : d;
+  if (!(m > 0x1p-300 && m < 0x1p300)) return 0x100u;
+  double e = fma(-d, y, 1.0);
+  if (e < 0) e = -e;
+  return e > 0x1p-54 ? 1u : 0u;
+}
+
+__device__ __noinline__ double ieee_quot(double v, double d) { return v / d; }
+// v / d, correctly rounded, from y = RN(1/d): Markstein's remainder step (IBM
+// J. Res. Dev. 34, 1990), a second one where q = RN(v y) may be more than an
+// ulp off (|1 - d y| > 2^-54).  A zero remainder leaves q as it is (its sign
+// too).  Numerators out of the range in which every intermediate is normal
+// take the division.
+__device__ __forceinline__ double div_any(double v, double d, double y, unsigned kind, int s) {
+  auto fix = [&](double q) {
+    const double r = fma(-q, d, v);
+    const double c = fma(r, y, q);
+    return (((unsigned)__double2hiint(r) << 1) | (unsigned)__double2loint(r)) ? c : q;
+  };
+  double q = fix(v * y);
+  if ((kind >> s) & 1u) q = fix(q);
+  const unsigned vh = (unsigned)__double2hiint(v) & 0x7fffffffu;
+  const bool usual = vh - 0x2d300000u < 0x25800000u || (vh | (unsigned)__double2loint(v)) == 0u;
+  if (!usual || ((kind >> (8 + s)) & 1u)) q = ieee_quot(v, d);
+  return q;
+}
 
 __device__ __forceinline__ bool adj_ok(const int8_t* c, const Dims& d, bool big, int i, int j, int k,
                                        int s) {
@@ -57,14 +119,6 @@ __device__ __forceinline__ FastF operator*(FastF a, FastF b) { return FastF(a.v 
 __device__ __forceinline__ FastF operator/(FastF a, FastF b) { return FastF(__fdividef(a.v, b.v)); }
 __device__ __forceinline__ FastF fabs(FastF a) { return FastF(fabsf(a.v)); }
 
-// a grid / coefficient value as T: the FP32 copy for the FP32 stencils, else
-// the FP64 table
-template <typename T>
-__device__ __forceinline__ T grid_t(const double* d64, const float* f32, int q) {
-  if constexpr (std::is_same<T, float>::value || std::is_same<T, FastF>::value) return T(f32[q]);
-  else return T(d64[q]);
-}
-
 // Forward-mode dual number (value, tangent): the stencil evaluated in it gives
 // the reference's FP64 value (the value part performs exactly the double
 // operations) and the exact derivative of the discrete stencil along the
@@ -79,10 +133,6 @@ __device__ __forceinline__ Dual operator+(Dual a, Dual b) { return Dual(a.v + b.
 __device__ __forceinline__ Dual operator-(Dual a, Dual b) { return Dual(a.v - b.v, a.d - b.d); }
 __device__ __forceinline__ Dual operator-(Dual a) { return Dual(-a.v, -a.d); }
 __device__ __forceinline__ Dual operator*(Dual a, Dual b) { return Dual(a.v * b.v, a.d * b.v + a.v * b.d); }
-__device__ __forceinline__ Dual operator/(Dual a, Dual b) {
-  const double q = a.v / b.v;
-  return Dual(q, (a.d - q * b.d) / b.v);
-}
 // |x| with the derivative of the branch the value takes (sign(0) = +); the
 // global float/double overloads stay visible next to it
 using ::fabs;
@@ -121,14 +171,91 @@ __device__ __forceinline__ Dual4 operator*(const Dual4& a, const Dual4& b) {
   for (int l = 0; l < 4; ++l) r.d[l] = a.d[l] * b.v + a.v * b.d[l];
   return r;
 }
-__device__ __forceinline__ Dual4 operator/(const Dual4& a, const Dual4& b) {
-  const double q = a.v / b.v;
-  Dual4 r(q);
+__device__ __forceinline__ Dual4 fabs(const Dual4& a) { return a.v < 0.0 ? -a : a; }
+
+// grid quantities have no tangent: plain numbers beside the dual types (the
+// tangent's zero products left out)
+template <typename T>
+struct GridNum {
+  using type = T;
+};
+template <>
+struct GridNum<Dual> {
+  using type = double;
+};
+template <>
+struct GridNum<Dual4> {
+  using type = double;
+};
+__device__ __forceinline__ Dual operator*(double c, Dual a) { return Dual(c * a.v, c * a.d); }
+__device__ __forceinline__ Dual4 operator*(double c, const Dual4& a) {
+  Dual4 r(c * a.v);
 #pragma unroll
-  for (int l = 0; l < 4; ++l) r.d[l] = (a.d[l] - q * b.d[l]) / b.v;
+  for (int l = 0; l < 4; ++l) r.d[l] = c * a.d[l];
   return r;
 }
-__device__ __forceinline__ Dual4 fabs(const Dual4& a) { return a.v < 0.0 ? -a : a; }
+
+// One axis's tables at one grid index.
+template <typename T>
+struct MomAxis {
+  static constexpr int n = 32;  // entries between slots
+  const double* t;
+  const float* f;
+  unsigned k;
+  __device__ __forceinline__ MomAxis(const DevBlock& B, int g0, int q)
+      : t(B.mt + mom_slot0(g0, q - 1, kMtSlots)), f(B.mtf + mom_slot0(g0, q - 1, kMfSlots)),
+        k(B.mtk[32 * g0 + q - 1]) {}
+  using G = typename GridNum<T>::type;
+  // numerator / divisor s: FP64 by div_any (the division's bits); FP32 of the
+  // mixed path by the reciprocal (the bits of __fdividef)
+  __device__ __forceinline__ T div(const T& a, int s) const {
+    if constexpr (std::is_same<T, FastF>::value) {
+      return FastF(a.v * f[s * n]);
+    } else if constexpr (std::is_same<T, float>::value) {
+      return a / f[(kMfD + s) * n];
+    } else {
+      const double d = t[2 * s * n], y = t[(2 * s + 1) * n];
+      if constexpr (std::is_same<T, double>::value) {
+        return div_any(a, d, y, k, s);
+      } else if constexpr (std::is_same<T, Dual>::value) {
+        return Dual(div_any(a.v, d, y, k, s), div_any(a.d, d, y, k, s));
+      } else {
+        Dual4 r(div_any(a.v, d, y, k, s));
+#pragma unroll
+        for (int l = 0; l < 4; ++l) r.d[l] = div_any(a.d[l], d, y, k, s);
+        return r;
+      }
+    }
+  }
+  __device__ __forceinline__ G quot(int s) const {
+    if constexpr (std::is_same<T, FastF>::value) return G(f[(kMfQ + s) * n]);
+    else if constexpr (std::is_same<T, float>::value) return f[(kMfI + s) * n];
+    else return t[(kMtQ + s) * n];
+  }
+  // column c (1..5) of CA (kind 0) / CK (1) self, CA (2) / CK (3) cross
+  __device__ __forceinline__ G coef(int kind, int c) const {
+    if constexpr (std::is_same<T, FastF>::value || std::is_same<T, float>::value)
+      return G(f[(kMfC + 5 * kind + c - 1) * n]);
+    else return t[(kMtC + 5 * kind + c - 1) * n];
+  }
+};
+
+// division by re
+template <typename T>
+__device__ __forceinline__ T div_re(const T& a, const MomArgs& m) {
+  if constexpr (std::is_same<T, double>::value) {
+    return div_any(a, m.re, m.re_y, m.re_k, 0);
+  } else if constexpr (std::is_same<T, Dual>::value) {
+    return Dual(div_any(a.v, m.re, m.re_y, m.re_k, 0), div_any(a.d, m.re, m.re_y, m.re_k, 0));
+  } else if constexpr (std::is_same<T, Dual4>::value) {
+    Dual4 r(div_any(a.v, m.re, m.re_y, m.re_k, 0));
+#pragma unroll
+    for (int l = 0; l < 4; ++l) r.d[l] = div_any(a.d[l], m.re, m.re_y, m.re_k, 0);
+    return r;
+  } else {
+    return a / T(m.re);
+  }
+}
 
 // where a stencil's three results go
 struct StoreOut {
@@ -153,6 +280,12 @@ struct PlainReader {
   __device__ __forceinline__ double get(int q, int, int, int, int64_t x) const { return __ldg(f[q] + x); }
 };
 
+// the FP32 copies of the fields (mixed path)
+struct PlainReaderF {
+  const float* f[4];
+  __device__ __forceinline__ float get(int q, int, int, int, int64_t x) const { return __ldg(f[q] + x); }
+};
+
 // One fluid cell (i,j,k) of nsMomentum2order.  T = double: the reference
 // arithmetic (bit-exact drop-in).  T = float: the FP32 momentum stencil of the
 // mixed-precision path (fields stay FP64 in HBM; stencil values are rounded to
@@ -160,10 +293,12 @@ struct PlainReader {
 template <typename T, class Rd, class Out>
 __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& a, int i, int j, int k,
                                               int64_t c, const Rd& rd, const Out& out) {
-  const T Q25 = T(0.25), HALF = T(0.5), TWO = T(2.0), ONE = T(1.0);
+  using G = typename GridNum<T>::type;
+  const G Q25 = G(0.25), HALF = G(0.5), alpha = G(1.0);
   const Dims& d = B.d;
-  const T alpha = ONE;
-  const T deltat = T(a.dt), re = T(a.re);
+  const G deltat = G(a.dt);
+  const int gy = mom_groups(d.NX), gz = gy + mom_groups(d.NY);
+  const MomAxis<T> AX(B, 0, i), AY(B, gy, j), AZ(B, gz, k);
   const int nx_var = d.nx, ny_var = d.ny, nz_var = d.nz;
   const int64_t SX = 1, SY = d.NX, SZ = (int64_t)d.NX * d.NY;
   {
@@ -171,15 +306,7 @@ __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& 
 #define v(a, b, e) (T) rd.get(1, i + (a), j + (b), k + (e), c + (a) * SX + (b) * SY + (e) * SZ)
 #define w(a, b, e) (T) rd.get(2, i + (a), j + (b), k + (e), c + (a) * SX + (b) * SY + (e) * SZ)
 #define p(a, b, e) (T) rd.get(3, i + (a), j + (b), k + (e), c + (a) * SX + (b) * SY + (e) * SZ)
-#define DX(q) grid_t<T>(B.dxa, B.dxf, (q) - 1)
-#define DY(q) grid_t<T>(B.dya, B.dyf, (q) - 1)
-#define DZ(q) grid_t<T>(B.dza, B.dzf, (q) - 1)
-#define CA(tab, row, q) grid_t<T>(B.ca[tab], B.caf[tab], ((row) - 1) + 6 * ((q) - 1))
-#define CK(tab, row, q) grid_t<T>(B.ck[tab], B.ckf[tab], ((row) - 1) + 6 * ((q) - 1))
     // offsets are relative to (i,j,k): u(-1,0,0) is u(i-1,j,k)
-    const T dxr = DX(i + 1), dx = DX(i), dxl = DX(i - 1);
-    const T dye = DY(j + 1), dy = DY(j), dyw = DY(j - 1);
-    const T dzt = DZ(k + 1), dz = DZ(k), dzb = DZ(k - 1);
 
     const T u1a = u(-1, 0, 0) + u(0, 0, 0);
     const T u22 = u(-1, 0, 0) - u(0, 0, 0);
@@ -232,12 +359,9 @@ __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& 
     const T w15 = w(0, 0, 0) + w(0, 0, 1);
     const T w16 = w(0, 0, 0) - w(0, 0, 1);
 
-    const T dpdx = (p(0, 0, 0) - p(1, 0, 0)) / (HALF * (dxr + dx));
-    const T dpdy = (p(0, 0, 0) - p(0, 1, 0)) / (HALF * (dye + dy));
-    const T dpdz = (p(0, 0, 0) - p(0, 0, 1)) / (HALF * (dzt + dz));
-
-    const T dx2xr = dx + dxr, dx2xl = dx + dxl, dy2ye = dy + dye, dy2yw = dy + dyw,
-                 dz2zt = dz + dzt, dz2zb = dz + dzb;
+    const T dpdx = AX.div(p(0, 0, 0) - p(1, 0, 0), MD_HALF_R);
+    const T dpdy = AY.div(p(0, 0, 0) - p(0, 1, 0), MD_HALF_R);
+    const T dpdz = AZ.div(p(0, 0, 0) - p(0, 0, 1), MD_HALF_R);
 
     // superset of the three components' third-order index ranges; inside it
     // the distance-2 neighbours exist
@@ -248,181 +372,106 @@ __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& 
 
     // ---------------- U momentum ----------------
     {
-      const T vu_e = v(1, 0, 0) + (dxr / (dx2xr)) * (v(0, 0, 0) - v(1, 0, 0));
-      const T vu_w = v(1, -1, 0) + (dxr / (dx2xr)) * (v(0, -1, 0) - v(1, -1, 0));
+      const T vu_e = v(1, 0, 0) + AX.quot(MQ_R) * (v(0, 0, 0) - v(1, 0, 0));
+      const T vu_w = v(1, -1, 0) + AX.quot(MQ_R) * (v(0, -1, 0) - v(1, -1, 0));
       const T v_in_um = HALF * (vu_e + vu_w);
-      const T wu_n = w(1, 0, 0) + (dxr / (dx2xr)) * (w(0, 0, 0) - w(1, 0, 0));
-      const T wu_s = w(1, 0, -1) + (dxr / (dx2xr)) * (w(0, 0, -1) - w(1, 0, -1));
+      const T wu_n = w(1, 0, 0) + AX.quot(MQ_R) * (w(0, 0, 0) - w(1, 0, 0));
+      const T wu_s = w(1, 0, -1) + AX.quot(MQ_R) * (w(0, 0, -1) - w(1, 0, -1));
       const T w_in_um = HALF * (wu_n + wu_s);
       T duudx, dvudy, dwudz;
       const bool third = (i > 2 && i < nx_var && j > 2 && j < ny_var + 1 && k > 2 && k < nz_var + 1) &&
                          !near_ib && !near_ts2;
       if (third) {
-        const T ddy = HALF * (DY(j) + DY(j - 1));
-        const T ddye = HALF * (DY(j) + DY(j + 1));
-        const T ddz = HALF * (DZ(k) + DZ(k - 1));
-        const T ddzr = HALF * (DZ(k) + DZ(k + 1));
-        duudx = u(0, 0, 0) *
-                    (CA(T_UU, 1, i) * u(2, 0, 0) + CA(T_UU, 2, i) * u(1, 0, 0) +
-                     CA(T_UU, 3, i) * u(0, 0, 0) + CA(T_UU, 4, i) * u(-1, 0, 0) +
-                     CA(T_UU, 5, i) * u(-2, 0, 0)) /
-                    (CA(T_UU, 6, i) * DX(i + 1)) +
-                fabs(u(0, 0, 0)) *
-                    (CK(T_UU, 1, i) * u(2, 0, 0) + CK(T_UU, 2, i) * u(1, 0, 0) +
-                     CK(T_UU, 3, i) * u(0, 0, 0) + CK(T_UU, 4, i) * u(-1, 0, 0) +
-                     CK(T_UU, 5, i) * u(-2, 0, 0)) /
-                    (TWO * CK(T_UU, 6, i) * DX(i));
-        dvudy = v_in_um *
-                    (CA(T_VU, 1, j) * u(0, 2, 0) + CA(T_VU, 2, j) * u(0, 1, 0) +
-                     CA(T_VU, 3, j) * u(0, 0, 0) + CA(T_VU, 4, j) * u(0, -1, 0) +
-                     CA(T_VU, 5, j) * u(0, -2, 0)) /
-                    (CA(T_VU, 6, j) * ddye) +
-                fabs(v_in_um) *
-                    (CK(T_VU, 1, j) * u(0, 2, 0) + CK(T_VU, 2, j) * u(0, 1, 0) +
-                     CK(T_VU, 3, j) * u(0, 0, 0) + CK(T_VU, 4, j) * u(0, -1, 0) +
-                     CK(T_VU, 5, j) * u(0, -2, 0)) /
-                    (TWO * CK(T_VU, 6, j) * ddy);
-        dwudz = w_in_um *
-                    (CA(T_WU, 1, k) * u(0, 0, 2) + CA(T_WU, 2, k) * u(0, 0, 1) +
-                     CA(T_WU, 3, k) * u(0, 0, 0) + CA(T_WU, 4, k) * u(0, 0, -1) +
-                     CA(T_WU, 5, k) * u(0, 0, -2)) /
-                    (CA(T_WU, 6, k) * ddzr) +
-                fabs(w_in_um) *
-                    (CK(T_WU, 1, k) * u(0, 0, 2) + CK(T_WU, 2, k) * u(0, 0, 1) +
-                     CK(T_WU, 3, k) * u(0, 0, 0) + CK(T_WU, 4, k) * u(0, 0, -1) +
-                     CK(T_WU, 5, k) * u(0, 0, -2)) /
-                    (TWO * CK(T_WU, 6, k) * ddz);
+        duudx =
+            AX.div(u(0, 0, 0) * (AX.coef(0, 1) * u(2, 0, 0) + AX.coef(0, 2) * u(1, 0, 0) + AX.coef(0, 3) * u(0, 0, 0) + AX.coef(0, 4) * u(-1, 0, 0) + AX.coef(0, 5) * u(-2, 0, 0)), MD_SA) +
+            AX.div(fabs(u(0, 0, 0)) * (AX.coef(1, 1) * u(2, 0, 0) + AX.coef(1, 2) * u(1, 0, 0) + AX.coef(1, 3) * u(0, 0, 0) + AX.coef(1, 4) * u(-1, 0, 0) + AX.coef(1, 5) * u(-2, 0, 0)), MD_SK);
+        dvudy =
+            AY.div(v_in_um * (AY.coef(2, 1) * u(0, 2, 0) + AY.coef(2, 2) * u(0, 1, 0) + AY.coef(2, 3) * u(0, 0, 0) + AY.coef(2, 4) * u(0, -1, 0) + AY.coef(2, 5) * u(0, -2, 0)), MD_XA) +
+            AY.div(fabs(v_in_um) * (AY.coef(3, 1) * u(0, 2, 0) + AY.coef(3, 2) * u(0, 1, 0) + AY.coef(3, 3) * u(0, 0, 0) + AY.coef(3, 4) * u(0, -1, 0) + AY.coef(3, 5) * u(0, -2, 0)), MD_XK);
+        dwudz =
+            AZ.div(w_in_um * (AZ.coef(2, 1) * u(0, 0, 2) + AZ.coef(2, 2) * u(0, 0, 1) + AZ.coef(2, 3) * u(0, 0, 0) + AZ.coef(2, 4) * u(0, 0, -1) + AZ.coef(2, 5) * u(0, 0, -2)), MD_XA) +
+            AZ.div(fabs(w_in_um) * (AZ.coef(3, 1) * u(0, 0, 2) + AZ.coef(3, 2) * u(0, 0, 1) + AZ.coef(3, 3) * u(0, 0, 0) + AZ.coef(3, 4) * u(0, 0, -1) + AZ.coef(3, 5) * u(0, 0, -2)), MD_XK);
       } else {
-        duudx = -Q25 * (u1a * u1a + alpha * fabs(u1a) * u22 - u3 * u3 - alpha * fabs(u3) * u4) / DX(i);
-        dvudy = -Q25 * (v1a * u5 + alpha * fabs(v1a) * u6 - v22 * u7 - alpha * fabs(v22) * u8) / DY(j);
-        dwudz = -Q25 * (w1a * u9 + alpha * fabs(w1a) * u10 - w22 * u11 - alpha * fabs(w22) * u12) / DZ(k);
+        duudx = AX.div(-Q25 * (u1a * u1a + alpha * fabs(u1a) * u22 - u3 * u3 - alpha * fabs(u3) * u4), MD_D);
+        dvudy = AY.div(-Q25 * (v1a * u5 + alpha * fabs(v1a) * u6 - v22 * u7 - alpha * fabs(v22) * u8), MD_D);
+        dwudz = AZ.div(-Q25 * (w1a * u9 + alpha * fabs(w1a) * u10 - w22 * u11 - alpha * fabs(w22) * u12), MD_D);
       }
-      const T d2udx2 = (TWO / dx2xr) * ((-u4 / dxr) + (u22 / dx));
+      const T d2udx2 = AX.quot(MQ_2) * (AX.div(-u4, MD_R) + AX.div(u22, MD_D));
       const T d2udy2 =
-          (TWO / (HALF * (dy2ye + dy2yw))) * ((-u8 / (HALF * dy2ye)) + (u6 / (HALF * dy2yw)));
+          AY.quot(MQ_C) * (AY.div(-u8, MD_HALF_R) + AY.div(u6, MD_HALF_L));
       const T d2udz2 =
-          (TWO / (HALF * (dz2zt + dz2zb))) * ((-u12 / (HALF * dz2zt)) + (u10 / (HALF * dz2zb)));
-      const T xtt2 = (d2udx2 + d2udy2 + d2udz2) / re;
+          AZ.quot(MQ_C) * (AZ.div(-u12, MD_HALF_R) + AZ.div(u10, MD_HALF_L));
+      const T xtt2 = div_re(d2udx2 + d2udy2 + d2udz2, a);
       const T residu = (-duudx - dvudy - dwudz + xtt2);
       out.put(0, c, u(0, 0, 0) + deltat * (residu + dpdx));
     }
     // ---------------- V momentum ----------------
     {
-      const T uv_e = u(0, 1, 0) + (dye / (dy2ye)) * (u(0, 0, 0) - u(0, 1, 0));
-      const T uv_w = u(-1, 1, 0) + (dye / (dy2ye)) * (u(-1, 0, 0) - u(-1, 1, 0));
+      const T uv_e = u(0, 1, 0) + AY.quot(MQ_R) * (u(0, 0, 0) - u(0, 1, 0));
+      const T uv_w = u(-1, 1, 0) + AY.quot(MQ_R) * (u(-1, 0, 0) - u(-1, 1, 0));
       const T u_in_vm = HALF * (uv_e + uv_w);
-      const T wv_n = w(0, 1, 0) + (dye / (dy2ye)) * (w(0, 0, 0) - w(0, 1, 0));
-      const T wv_s = w(0, 1, -1) + (dye / (dy2ye)) * (w(0, 0, -1) - w(0, 1, -1));
+      const T wv_n = w(0, 1, 0) + AY.quot(MQ_R) * (w(0, 0, 0) - w(0, 1, 0));
+      const T wv_s = w(0, 1, -1) + AY.quot(MQ_R) * (w(0, 0, -1) - w(0, 1, -1));
       const T w_in_vm = HALF * (wv_n + wv_s);
       T duvdx, dvvdy, dwvdz;
       const bool third = (i > 2 && i < nx_var + 1 && j > 2 && j < ny_var && k > 2 && k < nz_var + 1) &&
                          !near_ib && !near_ts2;
       if (third) {
-        const T ddx = HALF * (DX(i) + DX(i - 1));
-        const T ddxr = HALF * (DX(i) + DX(i + 1));
-        const T ddz = HALF * (DZ(k) + DZ(k - 1));
-        const T ddzr = HALF * (DZ(k) + DZ(k + 1));
-        duvdx = u_in_vm *
-                    (CA(T_UW, 1, i) * v(2, 0, 0) + CA(T_UW, 2, i) * v(1, 0, 0) +
-                     CA(T_UW, 3, i) * v(0, 0, 0) + CA(T_UW, 4, i) * v(-1, 0, 0) +
-                     CA(T_UW, 5, i) * v(-2, 0, 0)) /
-                    (CA(T_UW, 6, i) * ddxr) +
-                fabs(u_in_vm) *
-                    (CK(T_UW, 1, i) * v(2, 0, 0) + CK(T_UW, 2, i) * v(1, 0, 0) +
-                     CK(T_UW, 3, i) * v(0, 0, 0) + CK(T_UW, 4, i) * v(-1, 0, 0) +
-                     CK(T_UW, 5, i) * v(-2, 0, 0)) /
-                    (TWO * CK(T_UW, 6, i) * ddx);
-        dvvdy = v(0, 0, 0) *
-                    (CA(T_VV, 1, j) * v(0, 2, 0) + CA(T_VV, 2, j) * v(0, 1, 0) +
-                     CA(T_VV, 3, j) * v(0, 0, 0) + CA(T_VV, 4, j) * v(0, -1, 0) +
-                     CA(T_VV, 5, j) * v(0, -2, 0)) /
-                    (CA(T_VV, 6, j) * DY(j + 1)) +
-                fabs(v(0, 0, 0)) *
-                    (CK(T_VV, 1, j) * v(0, 2, 0) + CK(T_VV, 2, j) * v(0, 1, 0) +
-                     CK(T_VV, 3, j) * v(0, 0, 0) + CK(T_VV, 4, j) * v(0, -1, 0) +
-                     CK(T_VV, 5, j) * v(0, -2, 0)) /
-                    (TWO * CK(T_VV, 6, j) * DY(j));
-        dwvdz = w_in_vm *
-                    (CA(T_WU, 1, k) * v(0, 0, 2) + CA(T_WU, 2, k) * v(0, 0, 1) +
-                     CA(T_WU, 3, k) * v(0, 0, 0) + CA(T_WU, 4, k) * v(0, 0, -1) +
-                     CA(T_WU, 5, k) * v(0, 0, -2)) /
-                    (CA(T_WU, 6, k) * ddzr) +
-                fabs(w_in_vm) *
-                    (CK(T_WU, 1, k) * v(0, 0, 2) + CK(T_WU, 2, k) * v(0, 0, 1) +
-                     CK(T_WU, 3, k) * v(0, 0, 0) + CK(T_WU, 4, k) * v(0, 0, -1) +
-                     CK(T_WU, 5, k) * v(0, 0, -2)) /
-                    (TWO * CK(T_WU, 6, k) * ddz);
+        duvdx =
+            AX.div(u_in_vm * (AX.coef(2, 1) * v(2, 0, 0) + AX.coef(2, 2) * v(1, 0, 0) + AX.coef(2, 3) * v(0, 0, 0) + AX.coef(2, 4) * v(-1, 0, 0) + AX.coef(2, 5) * v(-2, 0, 0)), MD_XA) +
+            AX.div(fabs(u_in_vm) * (AX.coef(3, 1) * v(2, 0, 0) + AX.coef(3, 2) * v(1, 0, 0) + AX.coef(3, 3) * v(0, 0, 0) + AX.coef(3, 4) * v(-1, 0, 0) + AX.coef(3, 5) * v(-2, 0, 0)), MD_XK);
+        dvvdy =
+            AY.div(v(0, 0, 0) * (AY.coef(0, 1) * v(0, 2, 0) + AY.coef(0, 2) * v(0, 1, 0) + AY.coef(0, 3) * v(0, 0, 0) + AY.coef(0, 4) * v(0, -1, 0) + AY.coef(0, 5) * v(0, -2, 0)), MD_SA) +
+            AY.div(fabs(v(0, 0, 0)) * (AY.coef(1, 1) * v(0, 2, 0) + AY.coef(1, 2) * v(0, 1, 0) + AY.coef(1, 3) * v(0, 0, 0) + AY.coef(1, 4) * v(0, -1, 0) + AY.coef(1, 5) * v(0, -2, 0)), MD_SK);
+        dwvdz =
+            AZ.div(w_in_vm * (AZ.coef(2, 1) * v(0, 0, 2) + AZ.coef(2, 2) * v(0, 0, 1) + AZ.coef(2, 3) * v(0, 0, 0) + AZ.coef(2, 4) * v(0, 0, -1) + AZ.coef(2, 5) * v(0, 0, -2)), MD_XA) +
+            AZ.div(fabs(w_in_vm) * (AZ.coef(3, 1) * v(0, 0, 2) + AZ.coef(3, 2) * v(0, 0, 1) + AZ.coef(3, 3) * v(0, 0, 0) + AZ.coef(3, 4) * v(0, 0, -1) + AZ.coef(3, 5) * v(0, 0, -2)), MD_XK);
       } else {
-        duvdx = -Q25 * (u13 * v3 + alpha * fabs(u13) * v4 - u14 * v5 - alpha * fabs(u14) * v6) / DX(i);
-        dvvdy = -Q25 * (v7 * v7 + alpha * fabs(v7) * v8 - v9 * v9 - alpha * fabs(v9) * v10) / DY(j);
-        dwvdz = -Q25 * (w3 * v11 + alpha * fabs(w3) * v12 - w4 * v13 - alpha * fabs(w4) * v14) / DZ(k);
+        duvdx = AX.div(-Q25 * (u13 * v3 + alpha * fabs(u13) * v4 - u14 * v5 - alpha * fabs(u14) * v6), MD_D);
+        dvvdy = AY.div(-Q25 * (v7 * v7 + alpha * fabs(v7) * v8 - v9 * v9 - alpha * fabs(v9) * v10), MD_D);
+        dwvdz = AZ.div(-Q25 * (w3 * v11 + alpha * fabs(w3) * v12 - w4 * v13 - alpha * fabs(w4) * v14), MD_D);
       }
       const T d2vdx2 =
-          (TWO / (HALF * (dx2xr + dx2xl))) * ((-v6 / (HALF * dx2xr)) + (v4 / (HALF * dx2xl)));
-      const T d2vdy2 = (TWO / dy2ye) * ((-v10 / dye) + (v8 / dy));
+          AX.quot(MQ_C) * (AX.div(-v6, MD_HALF_R) + AX.div(v4, MD_HALF_L));
+      const T d2vdy2 = AY.quot(MQ_2) * (AY.div(-v10, MD_R) + AY.div(v8, MD_D));
       const T d2vdz2 =
-          (TWO / (HALF * (dz2zt + dz2zb))) * ((-v14 / (HALF * dz2zt)) + (v12 / (HALF * dz2zb)));
-      const T ytt2 = (d2vdx2 + d2vdy2 + d2vdz2) / re;
+          AZ.quot(MQ_C) * (AZ.div(-v14, MD_HALF_R) + AZ.div(v12, MD_HALF_L));
+      const T ytt2 = div_re(d2vdx2 + d2vdy2 + d2vdz2, a);
       const T residv = (-duvdx - dvvdy - dwvdz + ytt2);
       out.put(1, c, v(0, 0, 0) + deltat * (residv + dpdy));
     }
     // ---------------- W momentum ----------------
     {
-      const T uw_e = u(0, 0, 1) + (dzt / (dz2zt)) * (u(0, 0, 0) - u(0, 0, 1));
-      const T uw_w = u(-1, 0, 1) + (dzt / (dz2zt)) * (u(-1, 0, 0) - u(-1, 0, 1));
+      const T uw_e = u(0, 0, 1) + AZ.quot(MQ_R) * (u(0, 0, 0) - u(0, 0, 1));
+      const T uw_w = u(-1, 0, 1) + AZ.quot(MQ_R) * (u(-1, 0, 0) - u(-1, 0, 1));
       const T u_in_wm = HALF * (uw_e + uw_w);
-      const T vw_n = v(0, 0, 1) + (dzt / (dz2zt)) * (v(0, 0, 0) - v(0, 0, 1));
-      const T vw_s = v(0, -1, 1) + (dzt / (dz2zt)) * (v(0, -1, 0) - v(0, -1, 1));
+      const T vw_n = v(0, 0, 1) + AZ.quot(MQ_R) * (v(0, 0, 0) - v(0, 0, 1));
+      const T vw_s = v(0, -1, 1) + AZ.quot(MQ_R) * (v(0, -1, 0) - v(0, -1, 1));
       const T v_in_wm = HALF * (vw_n + vw_s);
       T duwdx, dvwdy, dwwdz;
       const bool third = (i > 2 && i < nx_var + 1 && j > 2 && j < ny_var + 1 && k > 2 && k < nz_var) &&
                          !near_ib && !near_ts2;
       if (third) {
-        const T ddx = HALF * (DX(i) + DX(i - 1));
-        const T ddxr = HALF * (DX(i) + DX(i + 1));
-        const T ddy = HALF * (DY(j) + DY(j - 1));
-        const T ddye = HALF * (DY(j) + DY(j + 1));
-        duwdx = u_in_wm *
-                    (CA(T_UW, 1, i) * w(2, 0, 0) + CA(T_UW, 2, i) * w(1, 0, 0) +
-                     CA(T_UW, 3, i) * w(0, 0, 0) + CA(T_UW, 4, i) * w(-1, 0, 0) +
-                     CA(T_UW, 5, i) * w(-2, 0, 0)) /
-                    (CA(T_UW, 6, i) * ddxr) +
-                fabs(u_in_wm) *
-                    (CK(T_UW, 1, i) * w(2, 0, 0) + CK(T_UW, 2, i) * w(1, 0, 0) +
-                     CK(T_UW, 3, i) * w(0, 0, 0) + CK(T_UW, 4, i) * w(-1, 0, 0) +
-                     CK(T_UW, 5, i) * w(-2, 0, 0)) /
-                    (TWO * CK(T_UW, 6, i) * ddx);
-        dvwdy = v_in_wm *
-                    (CA(T_VW, 1, j) * w(0, 2, 0) + CA(T_VW, 2, j) * w(0, 1, 0) +
-                     CA(T_VW, 3, j) * w(0, 0, 0) + CA(T_VW, 4, j) * w(0, -1, 0) +
-                     CA(T_VW, 5, j) * w(0, -2, 0)) /
-                    (CA(T_VW, 6, j) * ddye) +
-                fabs(v_in_wm) *
-                    (CK(T_VW, 1, j) * w(0, 2, 0) + CK(T_VW, 2, j) * w(0, 1, 0) +
-                     CK(T_VW, 3, j) * w(0, 0, 0) + CK(T_VW, 4, j) * w(0, -1, 0) +
-                     CK(T_VW, 5, j) * w(0, -2, 0)) /
-                    (TWO * CK(T_VW, 6, j) * ddy);
-        dwwdz = w(0, 0, 0) *
-                    (CA(T_WW, 1, k) * w(0, 0, 2) + CA(T_WW, 2, k) * w(0, 0, 1) +
-                     CA(T_WW, 3, k) * w(0, 0, 0) + CA(T_WW, 4, k) * w(0, 0, -1) +
-                     CA(T_WW, 5, k) * w(0, 0, -2)) /
-                    (CA(T_WW, 6, k) * DZ(k + 1)) +
-                fabs(w(0, 0, 0)) *
-                    (CK(T_WW, 1, k) * w(0, 0, 2) + CK(T_WW, 2, k) * w(0, 0, 1) +
-                     CK(T_WW, 3, k) * w(0, 0, 0) + CK(T_WW, 4, k) * w(0, 0, -1) +
-                     CK(T_WW, 5, k) * w(0, 0, -2)) /
-                    (TWO * CK(T_WW, 6, k) * DZ(k));
+        duwdx =
+            AX.div(u_in_wm * (AX.coef(2, 1) * w(2, 0, 0) + AX.coef(2, 2) * w(1, 0, 0) + AX.coef(2, 3) * w(0, 0, 0) + AX.coef(2, 4) * w(-1, 0, 0) + AX.coef(2, 5) * w(-2, 0, 0)), MD_XA) +
+            AX.div(fabs(u_in_wm) * (AX.coef(3, 1) * w(2, 0, 0) + AX.coef(3, 2) * w(1, 0, 0) + AX.coef(3, 3) * w(0, 0, 0) + AX.coef(3, 4) * w(-1, 0, 0) + AX.coef(3, 5) * w(-2, 0, 0)), MD_XK);
+        dvwdy =
+            AY.div(v_in_wm * (AY.coef(2, 1) * w(0, 2, 0) + AY.coef(2, 2) * w(0, 1, 0) + AY.coef(2, 3) * w(0, 0, 0) + AY.coef(2, 4) * w(0, -1, 0) + AY.coef(2, 5) * w(0, -2, 0)), MD_XA) +
+            AY.div(fabs(v_in_wm) * (AY.coef(3, 1) * w(0, 2, 0) + AY.coef(3, 2) * w(0, 1, 0) + AY.coef(3, 3) * w(0, 0, 0) + AY.coef(3, 4) * w(0, -1, 0) + AY.coef(3, 5) * w(0, -2, 0)), MD_XK);
+        dwwdz =
+            AZ.div(w(0, 0, 0) * (AZ.coef(0, 1) * w(0, 0, 2) + AZ.coef(0, 2) * w(0, 0, 1) + AZ.coef(0, 3) * w(0, 0, 0) + AZ.coef(0, 4) * w(0, 0, -1) + AZ.coef(0, 5) * w(0, 0, -2)), MD_SA) +
+            AZ.div(fabs(w(0, 0, 0)) * (AZ.coef(1, 1) * w(0, 0, 2) + AZ.coef(1, 2) * w(0, 0, 1) + AZ.coef(1, 3) * w(0, 0, 0) + AZ.coef(1, 4) * w(0, 0, -1) + AZ.coef(1, 5) * w(0, 0, -2)), MD_SK);
       } else {
-        duwdx = -HALF * (u15 * w5 + alpha * fabs(u15) * w6 - u16 * w7 - alpha * fabs(u16) * w8) / DX(i);
-        dvwdy = -HALF * (v15 * w9 + alpha * fabs(v15) * w10 - v16 * w11 - alpha * fabs(v16) * w12) / DY(j);
-        dwwdz = -HALF * (w13 * w13 + alpha * fabs(w13) * w14 - w15 * w15 - alpha * fabs(w15) * w16) / DZ(k);
+        duwdx = AX.div(-HALF * (u15 * w5 + alpha * fabs(u15) * w6 - u16 * w7 - alpha * fabs(u16) * w8), MD_D);
+        dvwdy = AY.div(-HALF * (v15 * w9 + alpha * fabs(v15) * w10 - v16 * w11 - alpha * fabs(v16) * w12), MD_D);
+        dwwdz = AZ.div(-HALF * (w13 * w13 + alpha * fabs(w13) * w14 - w15 * w15 - alpha * fabs(w15) * w16), MD_D);
       }
       const T d2wdx2 =
-          (TWO / (HALF * (dx2xr + dx2xl))) * ((-w8 / (HALF * dx2xr)) + (w6 / (HALF * dx2xl)));
+          AX.quot(MQ_C) * (AX.div(-w8, MD_HALF_R) + AX.div(w6, MD_HALF_L));
       const T d2wdy2 =
-          (TWO / (HALF * (dy2ye + dy2yw))) * ((-w12 / (HALF * dy2ye)) + (w10 / (HALF * dy2yw)));
-      const T d2wdz2 = (TWO / dz2zt) * ((-w16 / dzt) + (w14 / dz));
-      const T ztt2 = (d2wdx2 + d2wdy2 + d2wdz2) / re;
+          AY.quot(MQ_C) * (AY.div(-w12, MD_HALF_R) + AY.div(w10, MD_HALF_L));
+      const T d2wdz2 = AZ.quot(MQ_2) * (AZ.div(-w16, MD_R) + AZ.div(w14, MD_D));
+      const T ztt2 = div_re(d2wdx2 + d2wdy2 + d2wdz2, a);
       const T residw = (-duwdx - dvwdy - dwwdz + ztt2);
       out.put(2, c, w(0, 0, 0) + deltat * (residw + dpdz));
     }
@@ -430,24 +479,38 @@ __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& 
 #undef v
 #undef w
 #undef p
-#undef DX
-#undef DY
-#undef DZ
-#undef CA
-#undef CK
   }
 }
 
 template <typename T>
 struct MomentumOp {
   MomArgs a;
+  __device__ __forceinline__ static auto reader(const DevBlock& B) {
+    if constexpr (std::is_same<T, FastF>::value) return PlainReaderF{{B.mf[0], B.mf[1], B.mf[2], B.mf[3]}};
+    else return PlainReader{{B.u, B.v, B.w, B.p}};
+  }
   __device__ void run(const DevBlock& B, int cta, int ncta) const {
-    const PlainReader rd{{B.u, B.v, B.w, B.p}};
+    const auto rd = reader(B);
     FOR_INTERIOR(B, cta, ncta) {
       INTERIOR_CELL(B);
       if (B.cell[c] != 0) continue;
       if (B.tsnear[c]) continue;  // done by MomentumTsOp
       momentum_cell<T>(B, a, i, j, k, c, rd, StoreOut{B.ut, B.vt, B.wt});
+    }
+  }
+};
+
+// u,v,w,p rounded to FP32 once per point: the FP32 stencil reads each value
+// about 77 times, and GB300 converts FP64 to FP32 in the FP64 pipe (two lanes
+// per cycle and SM), where those conversions alone took half of its time
+struct CvtOp {
+  __device__ void run(const DevBlock& B, int cta, int ncta) const {
+    const int64_t n = B.d.npts(), step = (int64_t)ncta * blockDim.x;
+    for (int64_t t = (int64_t)cta * blockDim.x + threadIdx.x; t < n; t += step) {
+      B.mf[0][t] = (float)B.u[t];
+      B.mf[1][t] = (float)B.v[t];
+      B.mf[2][t] = (float)B.w[t];
+      B.mf[3][t] = (float)B.p[t];
     }
   }
 };
@@ -611,31 +674,89 @@ __device__ void own_substitution(const DevBlock& B, int i, int j, int k, int nts
   }
 }
 
+// own_substitution of one cell by a whole warp, 32 entries at a time; lane 0
+// writes the entries to last[]
+__device__ __forceinline__ void own_substitution_warp(const DevBlock& B, int i, int j, int k, int nts, int* last) {
+  const int lane = threadIdx.x & 31;
+  const double X[N_KIND] = {B.x1[i], B.x1[i - 1], B.xp[i - 1], B.xp[i - 1], B.xp[i - 1], B.xp[i - 1], B.xp[i - 1]};
+  const double Y[N_KIND] = {B.yp[j - 1], B.yp[j - 1], B.y1[j], B.y1[j - 1], B.yp[j - 1], B.yp[j - 1], B.yp[j - 1]};
+  const double Z[N_KIND] = {B.zp[k - 1], B.zp[k - 1], B.zp[k - 1], B.zp[k - 1], B.z1[k], B.z1[k - 1], B.zp[k - 1]};
+  unsigned open = (1u << N_KIND) - 1u;
+  for (int base = nts - 1; base >= 0 && open; base -= 32) {
+    const int nn = base - lane;
+    const int bt = nn >= 0 ? B.ts_idx[nn] - 1 : 0;
+#pragma unroll
+    for (int K = 0; K < N_KIND; ++K) {
+      if (!(open & (1u << K))) continue;
+      bool hit = false;
+      if (nn >= 0) {
+        const int e = B.nel[nel_slot(K)][bt] - 1;
+        const double t = (X[K] - B.xcent[e]) * B.cosA[e] + (Y[K] - B.ycent[e]) * B.cosB[e] +
+                         (Z[K] - B.zcent[e]) * B.cosG[e];
+        hit = t < 0;
+      }
+      const unsigned hits = __ballot_sync(0xffffffffu, hit);
+      if (hits) {
+        if (lane == 0) last[K] = base - (__ffs(hits) - 1);
+        open &= ~(1u << K);
+      }
+    }
+  }
+  if (lane == 0)
+#pragma unroll
+    for (int K = 0; K < N_KIND; ++K)
+      if (open & (1u << K)) last[K] = -1;
+}
+
+// The cells near TS cells.  A CTA's cells next to one search their
+// substituting entries warp by warp before the stencils run: the search goes
+// back through the list until each kind has hit, mostly one entry but up to
+// thousands, and one thread per cell left the kernel waiting for its longest
+// search (256x192x192 plate block, 6709 entries: 3.35 -> 1.16 ms).
 template <typename T>
 struct MomentumTsOp {
   MomArgs a;
   __device__ void run(const DevBlock& B, int cta, int ncta) const {
-  const Dims& d = B.d;
-  const int nts = (int)min(B.cnt[C_TS], (int64_t)B.cap_ib);
-  FOR_INTERIOR(B, cta, ncta) {
-    INTERIOR_CELL(B);
-    if (B.cell[c] != 0 || !B.tsnear[c]) continue;
-    TsReader rd;
-    rd.B = &B;
-    rd.gi = i;
-    rd.gj = j;
-    rd.gk = k;
-    rd.glin = c;
-    restore_consts(B, nts, rd.rconst);
-    const bool adj = !adj_ok(B.cell2, d, true, i, j, k, 1);
-    if (adj) {
-      own_substitution(B, i, j, k, nts, rd.last);
-    } else {
+    constexpr int NT = 128;
+    __shared__ int s_last[NT][N_KIND], s_list[NT], s_n;
+    const Dims& d = B.d;
+    const int nts = (int)min(B.cnt[C_TS], (int64_t)B.cap_ib);
+    const int64_t n = (int64_t)d.nx * d.ny * d.nz;
+    auto cell_at = [&](int64_t t, int& i, int& j, int& k) {
+      i = 2 + (int)(t % d.nx);
+      const int64_t r = t / d.nx;
+      j = 2 + (int)(r % d.ny);
+      k = 2 + (int)(r / d.ny);
+    };
+    for (int64_t t0 = (int64_t)cta * NT; t0 < n; t0 += (int64_t)ncta * NT) {
+      const int64_t t = t0 + threadIdx.x;
+      int i = 2, j = 2, k = 2;
+      if (t < n) cell_at(t, i, j, k);
+      const int64_t c = d.idx(i, j, k);
+      const bool near = t < n && B.tsnear[c] && B.cell[c] == 0;
+      if (threadIdx.x == 0) s_n = 0;
+      if (!__syncthreads_or(near)) continue;
+      const bool adj = near && !adj_ok(B.cell2, d, true, i, j, k, 1);
+      if (adj) s_list[atomicAdd(&s_n, 1)] = threadIdx.x;
+      __syncthreads();
+      for (int q = threadIdx.x >> 5; q < s_n; q += NT / 32) {
+        int ci, cj, ck;
+        cell_at(t0 + s_list[q], ci, cj, ck);
+        own_substitution_warp(B, ci, cj, ck, nts, s_last[s_list[q]]);
+      }
+      __syncthreads();
+      if (!near) continue;
+      TsReader rd;
+      rd.B = &B;
+      rd.gi = i;
+      rd.gj = j;
+      rd.gk = k;
+      rd.glin = c;
+      restore_consts(B, nts, rd.rconst);
 #pragma unroll
-      for (int K = 0; K < N_KIND; ++K) rd.last[K] = -1;
+      for (int K = 0; K < N_KIND; ++K) rd.last[K] = adj ? s_last[threadIdx.x][K] : -1;
+      momentum_cell<T>(B, a, i, j, k, c, rd, StoreOut{B.ut, B.vt, B.wt});
     }
-    momentum_cell<T>(B, a, i, j, k, c, rd, StoreOut{B.ut, B.vt, B.wt});
-  }
   }
 };
 
@@ -1088,12 +1209,127 @@ __global__ void k_solid_bc(DevBlock B, int move) {
   }
 }
 
+
+// the stencil's tables from the spacings and the coefficient tables, with the
+// operations and the order the stencil's expressions have in each precision
+__global__ void k_mom_tables(DevBlock B, double* mt, float* mtf, unsigned* mtk) {
+  const Dims& D = B.d;
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t0 >= D.NX + D.NY + D.NZ) return;
+  const int ax = t0 < D.NX ? 0 : t0 < D.NX + D.NY ? 1 : 2;
+  const int first = ax == 0 ? 0 : ax == 1 ? D.NX : D.NX + D.NY, len = ax == 0 ? D.NX : ax == 1 ? D.NY : D.NZ;
+  const int gy = mom_groups(D.NX), g0 = ax == 0 ? 0 : ax == 1 ? gy : gy + mom_groups(D.NY);
+  const int q = t0 - first + 1;  // 1-based grid index
+  constexpr int N = 32;          // entries between slots
+  double* T = mt + mom_slot0(g0, q - 1, kMtSlots);
+  float* F = mtf + mom_slot0(g0, q - 1, kMfSlots);
+  mtk[32 * g0 + q - 1] = 0xffffu;
+  if (q < 2 || q > len - 1) return;  // no cell there
+  const double* dd = ax == 0 ? B.dxa : ax == 1 ? B.dya : B.dza;
+  const float* df = ax == 0 ? B.dxf : ax == 1 ? B.dyf : B.dzf;
+  const int self = ax == 0 ? T_UU : ax == 1 ? T_VV : T_WW, cross = ax == 0 ? T_UW : ax == 1 ? T_VU : T_WU;
+  const int64_t col = 6 * (int64_t)(q - 1);
+  auto fill = [&](auto half, const auto* dl_, const auto* ca, const auto* ck, const auto* xa, const auto* xk,
+                  auto* div) {
+    using R = decltype(half);
+    const R dl = dl_[q - 2], d = dl_[q - 1], dr = dl_[q], two = R(2.0);
+    div[MD_HALF_R] = half * (d + dr);
+    div[MD_HALF_L] = half * (d + dl);
+    div[MD_SA] = ca[col + 5] * dr;
+    div[MD_SK] = two * ck[col + 5] * d;
+    div[MD_XA] = xa[col + 5] * (half * (d + dr));
+    div[MD_XK] = two * xk[col + 5] * (half * (d + dl));
+    div[MD_D] = d;
+    div[MD_R] = dr;
+  };
+  double e[N_MD];
+  float f[N_MD];
+  fill(0.5, dd, B.ca[self], B.ck[self], B.ca[cross], B.ck[cross], e);
+  fill(0.5f, df, B.caf[self], B.ckf[self], B.caf[cross], B.ckf[cross], f);
+  unsigned kind = 0;
+  for (int s = 0; s < N_MD; ++s) {
+    const double y = 1.0 / e[s];
+    T[2 * s * N] = e[s];
+    T[(2 * s + 1) * N] = y;
+    kind |= div_kind(e[s], y) << s;
+    F[s * N] = __fdividef(1.0f, f[s]);
+    F[(kMfD + s) * N] = f[s];
+  }
+  mtk[32 * g0 + q - 1] = kind;
+  const double r2 = dd[q - 1] + dd[q], l2 = dd[q - 1] + dd[q - 2];
+  T[(kMtQ + MQ_R) * N] = dd[q] / r2;
+  T[(kMtQ + MQ_2) * N] = 2.0 / r2;
+  T[(kMtQ + MQ_C) * N] = 2.0 / (0.5 * (r2 + l2));
+  const float g2 = df[q - 1] + df[q], h2 = df[q - 1] + df[q - 2];
+  F[(kMfQ + MQ_R) * N] = __fdividef(df[q], g2);
+  F[(kMfQ + MQ_2) * N] = __fdividef(2.0f, g2);
+  F[(kMfQ + MQ_C) * N] = __fdividef(2.0f, 0.5f * (g2 + h2));
+  F[(kMfI + MQ_R) * N] = df[q] / g2;
+  F[(kMfI + MQ_2) * N] = 2.0f / g2;
+  F[(kMfI + MQ_C) * N] = 2.0f / (0.5f * (g2 + h2));
+  for (int c = 0; c < 5; ++c) {
+    T[(kMtC + c) * N] = B.ca[self][col + c];
+    T[(kMtC + 5 + c) * N] = B.ck[self][col + c];
+    T[(kMtC + 10 + c) * N] = B.ca[cross][col + c];
+    T[(kMtC + 15 + c) * N] = B.ck[cross][col + c];
+    F[(kMfC + c) * N] = B.caf[self][col + c];
+    F[(kMfC + 5 + c) * N] = B.ckf[self][col + c];
+    F[(kMfC + 10 + c) * N] = B.caf[cross][col + c];
+    F[(kMfC + 15 + c) * N] = B.ckf[cross][col + c];
+  }
+}
+
+MomArgs mom_args(double dt, double re) {
+  const double y = 1.0 / re;
+  return MomArgs{dt, re, y, div_kind(re, y)};
+}
+
 }  // namespace
 
+// (re)builds the momentum stencil's per-line tables; the block's grids and
+// coefficient tables are on the device
+int launch_momentum_tables(HostBlock* hb) {
+  const Dims& d = hb->d.d;
+  const size_t n = 32 * (size_t)(mom_groups(d.NX) + mom_groups(d.NY) + mom_groups(d.NZ));
+  if (!hb->d.mt) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, n * (kMtSlots * sizeof(double) + kMfSlots * sizeof(float) + sizeof(unsigned))) != cudaSuccess)
+      return BCFD_E_NOMEM;
+    hb->allocs.push_back(p);
+    double* t = static_cast<double*>(p);
+    float* f = reinterpret_cast<float*>(t + n * kMtSlots);
+    hb->d.mt = t;
+    hb->d.mtf = f;
+    hb->d.mtk = reinterpret_cast<unsigned*>(f + n * kMfSlots);
+  }
+  k_mom_tables<<<grid_for(d.NX + d.NY + d.NZ, 128), 128, 0, stream()>>>(hb->d, const_cast<double*>(hb->d.mt),
+                                                               const_cast<float*>(hb->d.mtf),
+                                                               const_cast<unsigned*>(hb->d.mtk));
+  BCFD_LAUNCHED();
+  return 0;
+}
+
+// the FP32 copies of u, v, w, p (a block's first mixed step)
+static int ensure_f32_fields(HostBlock* hb) {
+  if (hb->d.mf[0]) return 0;
+  // rows of an odd pitch start anywhere: one array after the other, each on a
+  // 256-byte boundary
+  const size_t n = ((size_t)hb->d.d.npts() + 63) & ~(size_t)63;
+  void* p = nullptr;
+  if (cudaMalloc(&p, 4 * n * sizeof(float)) != cudaSuccess) return BCFD_E_NOMEM;
+  hb->allocs.push_back(p);
+  for (int q = 0; q < 4; ++q) hb->d.mf[q] = static_cast<float*>(p) + q * n;
+  return 0;
+}
+
 int launch_momentum(const std::vector<HostBlock*>& hbs, double dt, double re, bool fp32) {
-  const MomArgs a{dt, re};
+  const MomArgs a = mom_args(dt, re);
   const unsigned cap = 1u << 20;
-  if (fp32) TRY_R((launch_op<MomentumOp<FastF>, 128>(hbs, MomentumOp<FastF>{a}, Extent::Interior, cap)));
+  if (fp32) {
+    for (HostBlock* hb : hbs) TRY_R(ensure_f32_fields(hb));
+    TRY_R((launch_op<CvtOp, 256>(hbs, CvtOp{}, Extent::Points, 152u * 32u)));
+    TRY_R((launch_op<MomentumOp<FastF>, 128>(hbs, MomentumOp<FastF>{a}, Extent::Interior, cap)));
+  }
   else TRY_R((launch_op<MomentumOp<double>, 128>(hbs, MomentumOp<double>{a}, Extent::Interior, cap)));
   // cells within reach of TS cells (none without surfaces 51/52), then the
   // values the reference's loop leaves at the TS positions
@@ -1139,7 +1375,7 @@ int launch_solid_bc(HostBlock* hb, bool move) {
 // derivative along (du,dv,dw,dp); device arrays of the block's point count
 int launch_momentum_tangent(HostBlock* hb, double dt, double re, const double* const du[4], double* const val[3],
                             double* const tan[3]) {
-  MomentumTlmOp op{MomArgs{dt, re}, {du[0], du[1], du[2], du[3]}, val[0], val[1], val[2], tan[0], tan[1], tan[2]};
+  MomentumTlmOp op{mom_args(dt, re), {du[0], du[1], du[2], du[3]}, val[0], val[1], val[2], tan[0], tan[1], tan[2]};
   k_one<MomentumTlmOp, 128><<<grid_for((int64_t)hb->d.d.nx * hb->d.d.ny * hb->d.d.nz, 128, 1u << 20), 128, 0,
                               stream()>>>(hb->d, op);
   BCFD_LAUNCHED();
@@ -1157,7 +1393,7 @@ int launch_momentum_tangent(HostBlock* hb, double dt, double re, const double* c
 // read); without it such cells set BCFD_E_STATE.
 int launch_momentum_adjoint(HostBlock* hb, double dt, double re, const double* const sb[3], double* const ab[4],
                             uint32_t* foot, const MomTsAdj* ts) {
-  const MomArgs a{dt, re};
+  const MomArgs a = mom_args(dt, re);
   const int64_t ni = (int64_t)hb->d.d.nx * hb->d.d.ny * hb->d.d.nz;
   const int* last = nullptr;
   if (ts) {
