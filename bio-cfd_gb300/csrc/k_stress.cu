@@ -245,15 +245,34 @@ __global__ void k_stress_scale(DevBlock B, const double* seed, double* scale) {
   scale[3] = seed[3] * 2.0 / aSy;
 }
 
-// w[c][pos] += coef over all elements, in element order (one thread)
-__global__ void k_stress_accum(int ne, const double* coef, const int64_t* pos, double* w, int64_t np) {
-  if (blockIdx.x || threadIdx.x) return;
-  for (int e = 0; e < ne; ++e)
-    for (int c = 0; c < 4; ++c)
-      for (int q = 0; q < 8; ++q) {
-        const int64_t r = 32 * (int64_t)e + 8 * c + q;
-        w[c * np + pos[r]] += coef[r];
-      }
+// w[c][pos] += coef over all elements, in element order: one warp, a lane per
+// (c, q) of an element (32 distinct locations: the eight corners of a cell in
+// each of the four fields), the next elements' coefficients loaded ahead; every
+// location sees the additions in the order of the serial loop (one thread took
+// 7.2 ms on the 48^3 sphere's elements, one warp 0.61 ms)
+__global__ void __launch_bounds__(32) k_stress_accum(int ne, const double* coef, const int64_t* pos, double* w,
+                                                     int64_t np) {
+  constexpr int kAhead = 8;
+  const int lane = threadIdx.x;
+  double* wc = w + (lane >> 3) * np;
+  double c[kAhead];
+  int64_t p[kAhead];
+  auto load = [&](int u, int e) {
+    if (e >= ne) return;
+    c[u] = coef[32 * (int64_t)e + lane];
+    p[u] = pos[32 * (int64_t)e + lane];
+  };
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) load(u, u);
+  for (int e0 = 0; e0 < ne; e0 += kAhead) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (e0 + u >= ne) break;
+      wc[p[u]] += c[u];
+      load(u, e0 + kAhead + u);
+      __syncwarp();
+    }
+  }
 }
 
 // fixed-order pairwise reduction by one CTA
