@@ -99,7 +99,7 @@ struct HostBlock {
   double lcoef_dt = 0.0;           // the deltat they were computed for (0: not computed)
   float* coef_f32 = nullptr;       // device Acx/Acy/Acz rounded to FP32
   float* pcf2 = nullptr;           // second FP32 correction buffer (both colours) of the temporal-blocked sweeps
-  unsigned long long* ll = nullptr;  // packet slots of the resident sweeps
+  unsigned long long *ll = nullptr, *ll64 = nullptr;  // packet slots of the resident FP32 and FP64 sweeps
   int64_t mk = 0, mkx1 = 0, mkx2 = 0;  // findDistnode's extreme surface nodes (1-based)
   // fine-block moves (src/Search.F90:997-1370): the last move and the index
   // ranges of the old (cpy) and new (cpy_mv) positions of the moved data,
@@ -121,7 +121,7 @@ struct HostBlock {
   int dc_variant = 0;
   int solve_threads = 0;           // threads per CTA of the tiled solves (0: 256)
   int solve_ctas_per_sm = 0;       // co-resident CTAs per SM cap (0: occupancy limit)
-  int solve_sync = 0;              // FP64 solve: 0 point-to-point, 1 grid-wide phase barriers
+  int solve_sync = 0;              // FP64 solve: 0 point-to-point, 1 grid-wide phase barriers, 2 resident
   int sor_rev = 0;                 // FP64 solve: black half-sweep first (adjoint solves)
   int dc_threads = 0;              // FP32 correction: threads per CTA (0: 256)
   int dc_ctas_per_sm = 0;          // FP32 correction: CTAs per SM cap (0: occupancy limit)
@@ -268,6 +268,8 @@ int launch_sor_set(const std::vector<HostBlock*>& hbs, int64_t itmax, double dt,
 bool tb_solve_fits(HostBlock* hb);
 bool zm_solve_fits(HostBlock* hb);
 bool res_solve_fits(HostBlock* hb);
+bool res64_solve_fits(HostBlock* hb);
+constexpr int kSyncResident = 2;  // HostBlock::solve_sync of the resident FP64 solve
 double mixed_omega_of(const HostBlock* hb);
 int launch_sor_mixed_set(const std::vector<HostBlock*>& hbs, int64_t itmax, double dt, double div_tol);
 // res_tol > 0: stop on the FP64 residual dt*max|b/dt - A pc| <= res_tol

@@ -22,7 +22,7 @@ namespace bcfd {
 namespace {
 
 struct Shape {
-  int threads, ctas_per_sm, sync;  // sync: FP64 0 neighbour / 1 grid; FP32 variant 1 grid / 3 neighbour,
+  int threads, ctas_per_sm, sync;  // sync: FP64 0 neighbour / 1 grid / 2 resident; FP32 variant 1 grid / 3 neighbour,
                                    // 4 temporal-blocked, 5 z-marching TMA
 };
 struct Tuned {
@@ -148,7 +148,8 @@ void apply(HostBlock* hb, const Shape& s, bool fp32) {
 }
 
 int tune_block(HostBlock* hb, Tuned* out) {
-  static const Shape c64[] = {{256, 0, 0}, {512, 0, 0}, {256, 0, 1}, {512, 0, 1}, {512, 1, 0}};
+  // sync 2: the resident solve
+  static const Shape c64[] = {{256, 0, 0}, {512, 0, 0}, {256, 0, 1}, {512, 0, 1}, {512, 1, 0}, {512, 0, kSyncResident}};
   // {256, 4, *} selects the 64-register instantiation of the FP32 solve
   // {512, 0, 4}: the temporal-blocked sweeps (small blocks)
   // {384, 0, 5}: the z-marching TMA sweeps (large blocks)
@@ -166,6 +167,7 @@ int tune_block(HostBlock* hb, Tuned* out) {
   float best = 1e30f, best64 = 1e30f;
   Shape b64 = c64[0], b32 = c32[0];
   for (const Shape& s : c64) {
+    if (s.sync == kSyncResident && !res64_solve_fits(hb)) continue;
     apply(hb, s, false);
     float ms = 0;
     if ((r = time_trial(hb, false, 5, &ms))) break;

@@ -422,6 +422,15 @@ __device__ __forceinline__ double take_slot(BlockStats* st, int c, int cta) {
   return v;
 }
 
+// residual-target mode: sweep pairs to the next residual check, from the
+// reduction over the last `pairs` pairs
+__device__ __forceinline__ int64_t next_gap(const SorArgs& a, double res, double res_prev, int64_t pairs) {
+  if (!(res_prev > 0.0 && res < res_prev && res > a.res_tol)) return 5;
+  const double per_pair = log(res / res_prev) / (double)pairs;  // < 0
+  const double need = log(a.res_tol / res) / per_pair;          // > 0
+  return (int64_t)fmin(64.0, fmax(5.0, ceil(need * 1.15) + 1.0));
+}
+
 // one half-sweep of the pair's first (FIRST = 1: red, or black for the
 // adjoint's order) or second colour
 template <int FIRST>
@@ -493,15 +502,9 @@ __device__ __forceinline__ void sor64_body(const DevBlock& B, const SorArgs& a, 
       derr4 = take_slot(st, check, cta);
       ++check;
       if (target_mode) {
-        int64_t gap = 5;
-        if (res_prev > 0.0 && derr4 < res_prev && derr4 > a.res_tol) {
-          const double per_pair = log(derr4 / res_prev) / (double)(it - it_prev);  // < 0
-          const double need = log(a.res_tol / derr4) / per_pair;                   // > 0
-          gap = (int64_t)fmin(64.0, fmax(5.0, ceil(need * 1.15) + 1.0));
-        }
+        next_check = it + next_gap(a, derr4, res_prev, it - it_prev);
         res_prev = derr4;
         it_prev = it;
-        next_check = it + gap;
       }
     }
     if (a.res_tol > 0.0 ? (derr4 <= a.res_tol) : (derr4 < a.epsi)) break;
@@ -1848,6 +1851,361 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sor_res(DevBlock B, DcArgs a
   }
 }
 
+// ---------------------------------------------------------------------------
+// Resident FP64 solve: as the resident FP32 sweeps, one CTA per SM keeps its
+// tile of pc (both colours and one row around it) in shared memory for the
+// whole solve, and neighbour tiles exchange edge rows as polled packets.  The
+// FP64 pipe bounds the update, so nothing is recomputed: the tiles exchange
+// after every half-sweep ({half of a value, half-sweep number} packets), edge
+// rows first, so that a row travels while the tile's inner rows are updated;
+// rhs, dg and dgi are read from L2 (24 bytes per update, far below its rate).
+// Gone are the phase barriers and polls on counters, which took longer than
+// the arithmetic on small blocks.  The arithmetic is tile_half64's.
+//
+// One packet buffer per colour is enough: a tile stores half-sweep n + 2 of a
+// colour after it has read all its neighbours' half-sweep n + 1, which they
+// stored after reading this colour's half-sweep n.
+// ---------------------------------------------------------------------------
+constexpr int kRes64Threads = 512;
+
+struct Res64Args {
+  int tj, tk, ntj, ntk;
+  int half;                   // threads per parity group
+  unsigned long long* ll[2];  // packets per colour, two per packed position
+};
+
+struct Res64Tile {
+  Tile t;
+  int nh, nxh, slots;
+  double* e[2];  // rows (jj, kk) of the tile from (-1, -1)
+  __device__ __forceinline__ int row(int jj, int kk) const { return (kk + 1) * (t.nj + 2) + jj + 1; }
+};
+
+// lists of rows (jj + 1 | kk + 1 << 8) per parity of j + k: edge rows, inner
+// rows; then the neighbours' rows
+enum Res64List { R6_EDGE = 0, R6_IN = 1, R6_HALO = 4, R6_COUNT = 5 };
+
+__host__ __device__ inline size_t res64_bytes(int nxh, int nj, int nk) {
+  const size_t rows = (size_t)(nj + 2) * (nk + 2);
+  return (2 * rows * nxh + 6) * sizeof(double) + (rows + 8) * sizeof(unsigned short);
+}
+
+__device__ __forceinline__ void write_pair(unsigned long long* slot, unsigned ph, double x, double y) {
+  ulonglong2* p = reinterpret_cast<ulonglong2*>(slot);
+  const unsigned long long hi = (unsigned long long)ph << 32;
+  st_packets(p, hi | (unsigned)__double2loint(x), hi | (unsigned)__double2hiint(x));
+  st_packets(p + 1, hi | (unsigned)__double2loint(y), hi | (unsigned)__double2hiint(y));
+}
+
+// colour c's rows around the tile, half-sweep `ph`; false: the wait gave up
+__device__ __forceinline__ bool res64_import(const DevBlock& B, const Res64Tile& R, const unsigned short* list, int n,
+                                             const unsigned long long* ll, double* e, unsigned ph, const GridBar& gb) {
+  constexpr int U = 2;
+  const int total = n * R.nh, nxh = R.nxh;
+  unsigned long long t0 = 0;
+  unsigned spins = 0;
+  for (int q0 = threadIdx.x; q0 < total; q0 += U * blockDim.x) {
+    const ulonglong2* p[U];
+    double2* dst[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * blockDim.x;
+      p[u] = nullptr;
+      if (q < total) {
+        const int r = q / R.nh, a = q - r * R.nh;
+        const int jj = (list[r] & 255) - 1, kk = (list[r] >> 8) - 1;
+        const int j = R.t.j0 + jj, k = R.t.k0 + kk;
+        p[u] = reinterpret_cast<const ulonglong2*>(
+            ll + 2 * ((int64_t)nxh * ((j - 1) + (int64_t)B.d.NY * (k - 1)) + 2 * a));
+        dst[u] = reinterpret_cast<double2*>(e + R.row(jj, kk) * nxh + 2 * a);
+      }
+    }
+    for (;;) {
+      ulonglong2 x[U], y[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (p[u]) {
+          x[u] = ld_packets(p[u]);
+          y[u] = ld_packets(p[u] + 1);
+        }
+      bool more = false;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (p[u]) {
+          if ((unsigned)(x[u].x >> 32) == ph && (unsigned)(x[u].y >> 32) == ph && (unsigned)(y[u].x >> 32) == ph &&
+              (unsigned)(y[u].y >> 32) == ph) {
+            *dst[u] = make_double2(__hiloint2double((int)x[u].y, (int)x[u].x),
+                                   __hiloint2double((int)y[u].y, (int)y[u].x));
+            p[u] = nullptr;
+          } else {
+            more = true;
+          }
+        }
+      if (!more) break;
+      if ((++spins & 63u) == 0) {
+        if (t0 == 0) t0 = globaltimer_ns();
+        if ((ld_relaxed_u64(gb.ctr) & kBarAbandon) || ld_acquire_i(gb.err) != 0) return false;
+        if (globaltimer_ns() - t0 > gb.limit_ns) {
+          atomicCAS(gb.err, 0, BCFD_E_TIMEOUT);
+          return false;
+        }
+      }
+    }
+  }
+  return true;
+}
+
+// one half-sweep of colour C over this thread's rows of a list, x-parity PAR
+// (WHAT 0: the reference's update, 1: without a division, 2: no update, lmax
+// takes the residual's magnitude); chk: lmax takes the increments' magnitudes
+template <int C, int PAR, int WHAT>
+__device__ __forceinline__ void res64_rows(const DevBlock& B, const Res64Args& z, const Res64Tile& R,
+                                           const unsigned short* list, int nedge, int n, int a, int slot, unsigned ph,
+                                           double omega, bool chk, unsigned long long& lmax) {
+  const int nxh = R.nxh, nj = R.t.nj, nk = R.t.nk, nx = B.d.nx;
+  const double* __restrict__ o = R.e[1 - C] + 2 * a;
+  double* __restrict__ own = R.e[C] + 2 * a;
+  const int sk = (nj + 2) * nxh;
+  const double om1 = 1.0 - omega;
+  // the pair's x coefficients, i clamped to the interior (cells outside are
+  // not updated)
+  const int i0 = 4 * a + 1 + PAR, c0 = min(max(i0, 2), nx + 1) - 2, c1 = min(max(i0 + 2, 2), nx + 1) - 2;
+  const double a1[2] = {B.Acx[c0], B.Acx[c1]}, a3[2] = {B.Acx[c0 + 2 * nx], B.Acx[c1 + 2 * nx]};
+  for (int q = slot; q < n; q += R.slots) {
+    const int jj = (list[q] & 255) - 1, kk = (list[q] >> 8) - 1;
+    const int j = R.t.j0 + jj, k = R.t.k0 + kk;
+    const int64_t pi = (int64_t)nxh * ((j - 1) + (int64_t)B.d.NY * (k - 1)) + 2 * a;
+    const uchar2 mk = *reinterpret_cast<const uchar2*>(B.upd[C] + pi);
+    const int w = R.row(jj, kk) * nxh;
+    const double2 x2 = *reinterpret_cast<const double2*>(own + w);
+    double nv[2] = {x2.x, x2.y};
+    if (mk.x | mk.y) {
+      const double2 b2 = *reinterpret_cast<const double2*>(B.rhs[C] + pi);
+      const double2 d2 = *reinterpret_cast<const double2*>(B.dg[C] + pi);
+      double2 s2 = make_double2(0.0, 0.0);
+      if (WHAT != 2) s2 = *reinterpret_cast<const double2*>(B.dgi[C] + pi);
+      const double2 oc = *reinterpret_cast<const double2*>(o + w), os = *reinterpret_cast<const double2*>(o + w - nxh);
+      const double2 on = *reinterpret_cast<const double2*>(o + w + nxh);
+      const double2 ob = *reinterpret_cast<const double2*>(o + w - sk), ot = *reinterpret_cast<const double2*>(o + w + sk);
+      const double ox = PAR ? o[w + 2] : o[w - 1];
+      const double ay1 = B.Acy[j - 2], ay3 = B.Acy[j - 2 + 2 * B.d.ny];
+      const double az1 = B.Acz[k - 2], az3 = B.Acz[k - 2 + 2 * B.d.nz];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const double left = u == 0 ? (PAR ? oc.x : ox) : (PAR ? oc.y : oc.x);
+        const double right = u == 0 ? (PAR ? oc.y : oc.x) : (PAR ? ox : oc.y);
+        const double old = nv[u], dg = u == 0 ? d2.x : d2.y, si = u == 0 ? s2.x : s2.y;
+        const double ps = u == 0 ? os.x : os.y, pn = u == 0 ? on.x : on.y;
+        const double pb = u == 0 ? ob.x : ob.y, pt = u == 0 ? ot.x : ot.y;
+        double v = u == 0 ? b2.x : b2.y;
+        if (WHAT == 2) {
+          double ax = dg * old;
+          ax = fma(a1[u], left, ax);
+          ax = fma(a3[u], right, ax);
+          ax = fma(ay1, ps, ax);
+          ax = fma(ay3, pn, ax);
+          ax = fma(az1, pb, ax);
+          ax = fma(az3, pt, ax);
+          v = v - ax;
+          if (u == 0 ? mk.x : mk.y) lmax = max(lmax, (unsigned long long)__double_as_longlong(fabs(v)));
+          continue;
+        }
+        if (WHAT == 1) {
+          v = fma(-dg, old, v);
+          v = fma(-a1[u], left, v);
+          v = fma(-a3[u], right, v);
+          v = fma(-ay1, ps, v);
+          v = fma(-ay3, pn, v);
+          v = fma(-az1, pb, v);
+          v = fma(-az3, pt, v);
+          v = fma(si, v, old);
+        } else {
+          v = v - a1[u] * left - a3[u] * right - ay1 * ps - ay3 * pn - az1 * pb - az3 * pt;
+          v = om1 * old + omega * div_by(v, dg, si);
+        }
+        if (u == 0 ? mk.x : mk.y) {
+          nv[u] = v;
+          if (chk) lmax = max(lmax, (unsigned long long)__double_as_longlong(fabs(v - old)));
+        }
+      }
+    }
+    if (WHAT == 2) continue;
+    *reinterpret_cast<double2*>(own + w) = make_double2(nv[0], nv[1]);
+    if (q < nedge) write_pair(z.ll[C] + 2 * pi, ph, nv[0], nv[1]);
+  }
+}
+
+__global__ void __launch_bounds__(kRes64Threads, 1) k_sor64_res(DevBlock B, SorArgs a, GridBar gb, Res64Args z) {
+  extern __shared__ float4 res_raw[];
+  __shared__ double sh[32];
+  __shared__ int cnt[R6_COUNT], off[R6_COUNT];
+  const Dims& d = B.d;
+  const int cta = (int)blockIdx.x;
+  Res64Tile R;
+  R.t = my_tile(d, TileMap{z.tj, z.tk, z.ntj, z.ntk, nullptr, 1}, cta);
+  R.nxh = d.NXH;
+  R.nh = d.NXH >> 1;
+  R.slots = z.half / R.nh;
+  const int nj = R.t.nj, nk = R.t.nk, nh = R.nh, rows = (nj + 2) * (nk + 2);
+  R.e[0] = reinterpret_cast<double*>(res_raw) + 2;
+  R.e[1] = R.e[0] + rows * R.nxh + 2;
+  unsigned short* const lists = reinterpret_cast<unsigned short*>(R.e[1] + rows * R.nxh + 2);
+  auto each_row = [&](auto&& put) {
+    for (int q = threadIdx.x; q < rows; q += blockDim.x) {
+      const int jj = q % (nj + 2) - 1, kk = q / (nj + 2) - 1, j = R.t.j0 + jj, k = R.t.k0 + kk;
+      if (j < 2 || j > d.ny + 1 || k < 2 || k > d.nz + 1) continue;  // ghost rows keep their values
+      const bool oj = jj < 0 || jj >= nj, ok = kk < 0 || kk >= nk;
+      const unsigned short v = (unsigned short)((jj + 1) | ((kk + 1) << 8));
+      if (oj && ok) continue;  // not a face neighbour
+      if (oj || ok) {
+        put(R6_HALO, v);
+        continue;
+      }
+      const bool edge = (jj == 0 && R.t.a > 0) || (jj == nj - 1 && R.t.a + 1 < z.ntj) || (kk == 0 && R.t.b > 0) ||
+                        (kk == nk - 1 && R.t.b + 1 < z.ntk);
+      put(2 * ((j + k) & 1) + (edge ? R6_EDGE : R6_IN), v);
+    }
+  };
+  if (threadIdx.x < R6_COUNT) cnt[threadIdx.x] = 0;
+  __syncthreads();
+  each_row([&](int l, unsigned short) { atomicAdd(&cnt[l], 1); });
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int at = 0;
+    for (int l = 0; l < R6_COUNT; ++l) {
+      off[l] = at;
+      at += cnt[l];
+      cnt[l] = 0;
+    }
+  }
+  __syncthreads();
+  each_row([&](int l, unsigned short v) { lists[off[l] + atomicAdd(&cnt[l], 1)] = v; });
+  // pc of the tile and the rows around it
+  for (int q = threadIdx.x; q < rows * nh; q += blockDim.x) {
+    const int r = q / nh, ra = q - r * nh;
+    const int jj = r % (nj + 2) - 1, kk = r / (nj + 2) - 1;
+    const int64_t pi = (int64_t)R.nxh * ((R.t.j0 + jj - 1) + (int64_t)d.NY * (R.t.k0 + kk - 1)) + 2 * ra;
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      *reinterpret_cast<double2*>(R.e[c] + 2 * q) = *reinterpret_cast<const double2*>(B.pc[c] + pi);
+  }
+  const bool odd = (int)threadIdx.x >= z.half;
+  const int lt = (int)threadIdx.x - (odd ? z.half : 0);
+  const int pa = lt % nh, slot = lt / nh < R.slots ? lt / nh : 0x40000000;
+  BlockStats* st = B.stats;
+  const int64_t it0 = st->niter;
+  // every CTA has read niter before CTA 0 may rewrite it at the end
+  if (!grid_sync(gb)) return;
+  int64_t it = it0;
+  int r5 = (int)(it0 % 5);
+  double derr4 = 11111.0;
+  int check = 0;
+  unsigned ph = 0;
+  bool ok = true;
+  const bool target_mode = a.res_tol > 0.0;
+  int64_t next_check = it0 + 5, it_prev = it0;
+  double res_prev = -1.0;
+  unsigned have[2] = {0, 0};  // half-sweep whose rows of each colour the halo holds
+  unsigned done[2] = {0, 0};  // last half-sweep of each colour
+  // the rows of colour c around the tile, if they changed since the last time
+  auto bring = [&](int c) -> bool {
+    bool got = true;
+    const unsigned want = c ? done[1] : done[0];
+    if (want != (c ? have[1] : have[0]))
+      got = res64_import(B, R, lists + off[R6_HALO], cnt[R6_HALO], c ? z.ll[1] : z.ll[0], c ? R.e[1] : R.e[0], want, gb);
+    if (c) have[1] = want;
+    else have[0] = want;
+    return !__syncthreads_or(!got);
+  };
+  unsigned long long lbits = 0;
+  // rows of this thread's group: colour c at x-parity PAR has j + k of parity
+  // PAR ^ c ^ 1
+  auto half_sweep = [&](int c, bool chk) -> bool {
+    const int l = 2 * ((odd ? 1 : 0) ^ c ^ 1), ne = cnt[l], n = ne + cnt[l + 1];
+    const unsigned short* list = lists + off[l];
+    if (!bring(1 - c)) return false;
+    ++ph;
+    if (c) done[1] = ph;
+    else done[0] = ph;
+    if (a.fast) {
+      if (c) {
+        if (odd) res64_rows<1, 1, 1>(B, z, R, list, ne, n, pa, slot, ph, a.omega, chk, lbits);
+        else res64_rows<1, 0, 1>(B, z, R, list, ne, n, pa, slot, ph, a.omega, chk, lbits);
+      } else {
+        if (odd) res64_rows<0, 1, 1>(B, z, R, list, ne, n, pa, slot, ph, a.omega, chk, lbits);
+        else res64_rows<0, 0, 1>(B, z, R, list, ne, n, pa, slot, ph, a.omega, chk, lbits);
+      }
+    } else {
+      if (c) {
+        if (odd) res64_rows<1, 1, 0>(B, z, R, list, ne, n, pa, slot, ph, a.omega, chk, lbits);
+        else res64_rows<1, 0, 0>(B, z, R, list, ne, n, pa, slot, ph, a.omega, chk, lbits);
+      } else {
+        if (odd) res64_rows<0, 1, 0>(B, z, R, list, ne, n, pa, slot, ph, a.omega, chk, lbits);
+        else res64_rows<0, 0, 0>(B, z, R, list, ne, n, pa, slot, ph, a.omega, chk, lbits);
+      }
+    }
+    return true;
+  };
+  for (;;) {
+    ++it;
+    if (++r5 == 5) r5 = 0;
+    const bool chk = !target_mode && r5 == 0;
+    lbits = 0;
+    const int first = a.rev ? 0 : 1;
+    if (!half_sweep(first, chk) || !half_sweep(1 - first, chk)) { ok = false; break; }
+    if (target_mode ? it >= next_check : r5 == 0) {
+      double lmax;
+      if (target_mode) {
+        if (!bring(1 - first)) { ok = false; break; }
+        lbits = 0;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int l = 2 * ((odd ? 1 : 0) ^ c ^ 1), n = cnt[l] + cnt[l + 1];
+          const unsigned short* list = lists + off[l];
+          if (c) {
+            if (odd) res64_rows<1, 1, 2>(B, z, R, list, 0, n, pa, slot, 0, 0.0, false, lbits);
+            else res64_rows<1, 0, 2>(B, z, R, list, 0, n, pa, slot, 0, 0.0, false, lbits);
+          } else {
+            if (odd) res64_rows<0, 1, 2>(B, z, R, list, 0, n, pa, slot, 0, 0.0, false, lbits);
+            else res64_rows<0, 0, 2>(B, z, R, list, 0, n, pa, slot, 0, 0.0, false, lbits);
+          }
+        }
+        lmax = __longlong_as_double((long long)lbits) * a.dt;
+      } else {
+        lmax = __longlong_as_double((long long)lbits);
+      }
+      const double m = block_max(lmax, sh);
+      if (threadIdx.x == 0) atomic_max_nonneg(&st->slot[check % 3], m);
+      if (!grid_sync(gb)) { ok = false; break; }
+      derr4 = take_slot(st, check, cta);
+      ++check;
+      if (target_mode) next_check = it + next_gap(a, derr4, res_prev, it - it_prev), res_prev = derr4, it_prev = it;
+    }
+    if (a.res_tol > 0.0 ? (derr4 <= a.res_tol) : (derr4 < a.epsi)) break;
+    if (it > a.itmax || non_finite(derr4)) break;
+  }
+  if (!ok && threadIdx.x == 0) atomicOr(gb.ctr, kBarAbandon);
+  // the tile back to pc
+  __syncthreads();
+  {
+    Walk3 w;
+    w.init(threadIdx.x, blockDim.x, nh, nj);
+    for (int q = threadIdx.x; q < nh * nj * nk; q += blockDim.x, w.next()) {
+      const int64_t pi = (int64_t)R.nxh * ((R.t.j0 + w.b - 1) + (int64_t)d.NY * (R.t.k0 + w.c - 1)) + 2 * w.a;
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        *reinterpret_cast<double2*>(B.pc[c] + pi) =
+            *reinterpret_cast<const double2*>(R.e[c] + R.row(w.b, w.c) * R.nxh + 2 * w.a);
+    }
+  }
+  if (cta == 0 && threadIdx.x == 0) {
+    log_solve(a.log, it - it0, 0, B.cnt[C_FLUID], 0);
+    st->niter = it;
+    st->derr2 = derr4;
+    if (ok && non_finite(derr4)) set_err(B.err, BCFD_E_NONFINITE);
+  }
+}
+
 // Several blocks' solves in one cooperative launch: member m owns CTAs
 // [cta0, cta0 + its tile count) and has its own barrier, tiles and slots.
 constexpr int kMaxSolveBatch = 16;
@@ -2193,9 +2551,92 @@ static int launch_rhs(HostBlock* hb, double dt, int fast) {
   return 0;
 }
 
+// Resident FP64 solve: the tile that gives the fullest SM the fewest rows (the
+// FP64 pipe's time), squarest among equals; 0 when it does not fit
+static int res64_shape(HostBlock* hb, Res64Args* z, size_t* bytes) {
+  const Dims& d = hb->d.d;
+  const int nh = d.NXH / 2;
+  if (nh > kRes64Threads / 2) return 0;
+  int smem_max = 0;
+  if (cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, lib().device) != cudaSuccess)
+    return 0;
+  const int nsm = num_sms();
+  long best = -1;
+  int per = 0;
+  for (int ntj = 1; ntj <= std::min(d.ny, nsm); ++ntj) {
+    const int tj = (d.ny + ntj - 1) / ntj;
+    if ((d.ny + tj - 1) / tj != ntj || tj > 250) continue;
+    const int ntk0 = std::min(d.nz, nsm / ntj);
+    const int tk = (d.nz + ntk0 - 1) / ntk0, ntk = (d.nz + tk - 1) / tk;
+    if (tk > 250) continue;
+    const long rows = (long)tj * tk;
+    if (best < 0 || rows < best || (rows == best && tj + tk < per)) {
+      best = rows;
+      per = tj + tk;
+      z->tj = tj;
+      z->ntj = ntj;
+      z->tk = tk;
+      z->ntk = ntk;
+    }
+  }
+  if (best < 0) return 0;
+  *bytes = res64_bytes(d.NXH, z->tj, z->tk);
+  if (*bytes > (size_t)smem_max - 1024) return 0;  // static shared memory of the kernel
+  const int lines = std::max(1, std::min(kRes64Threads / 2 / nh, (int)((best + 1) / 2)));
+  z->half = std::min(kRes64Threads / 2, (lines * nh + 31) / 32 * 32);
+  return 1;
+}
+
+bool res64_solve_fits(HostBlock* hb) {
+  Res64Args z{};
+  size_t bytes = 0;
+  return res64_shape(hb, &z, &bytes) != 0;
+}
+
+static int launch_sor64_res(HostBlock* hb, SorArgs a) {
+  DevBlock& B = hb->d;
+  Res64Args z{};
+  size_t smem = 0;
+  if (!res64_shape(hb, &z, &smem)) return BCFD_E_STATE;
+  const size_t np = (size_t)B.d.npacked(), llb = 4 * np * sizeof(unsigned long long);
+  if (!hb->ll64) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, llb) != cudaSuccess) return BCFD_E_NOMEM;
+    hb->allocs.push_back(p);
+    hb->ll64 = static_cast<unsigned long long*>(p);
+    lib().gen++;
+  }
+  BCFD_CUDA(cudaMemsetAsync(hb->ll64, 0, llb, stream()));
+  z.ll[0] = hb->ll64;
+  z.ll[1] = hb->ll64 + 2 * np;
+  TRY_R(reset_solve_state(hb, TileMap{z.tj, z.tk, z.ntj, z.ntk, hb->prog, 1}));
+  BCFD_CUDA(cudaFuncSetAttribute((const void*)k_sor64_res, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const unsigned grid = (unsigned)(z.ntj * z.ntk);
+  GridBar gb = make_bar(B.err, grid);
+  gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
+  void* args[] = {(void*)&B, (void*)&a, (void*)&gb, (void*)&z};
+  prof_mark(true);
+  BCFD_CUDA(launch_coop((const void*)k_sor64_res, grid, (unsigned)(2 * z.half), args, smem));
+  prof_mark(false);
+  BCFD_LAUNCHED();
+  return 0;
+}
+
 int launch_sor(HostBlock* hb, int64_t itmax, double dt, double epsi, double res_tol, int fast) {
   DevBlock& B = hb->d;
   TRY_R(launch_rhs(hb, dt, fast));
+  // the resident solve by the autotuner's choice, or by default (no launch
+  // shape asked for) on blocks of up to kRes64Cells cells, where the phase
+  // barriers outweigh the arithmetic: per sweep pair, tiled -> resident, 10.4
+  // -> 6.5 us on 20^3, 11.3 -> 8.1 on 40^3, 15.6 -> 12.8 on 56^3, but 19.6 ->
+  // 21.1 on 64^3 (one CTA per SM fills the FP64 pipe less evenly than three)
+  const bool shaped = hb->solve_threads > 0 || hb->solve_sync != 0 || hb->solve_ctas_per_sm > 0;
+  constexpr int64_t kRes64Cells = 200000;
+  const bool small = (int64_t)B.d.nx * B.d.ny * B.d.nz <= kRes64Cells;
+  if ((hb->solve_sync == kSyncResident || (!shaped && small)) && res64_solve_fits(hb)) {
+    TRY_R(launch_sor64_res(hb, SorArgs{itmax, epsi, hb->omega, prof_log(), res_tol, dt, hb->sor_rev, fast}));
+    return launch_residual(hb, dt);
+  }
   const int threads = hb->solve_threads > 0 ? hb->solve_threads : kSor64Threads;
   const void* fn = threads > 256 ? (const void*)k_sor64<kSolveMaxThreads> : (const void*)k_sor64<256>;
   TileMap tm = choose_tiles(hb, fn, threads, hb->solve_sync == 1 ? 1 : 0, hb->solve_ctas_per_sm);

@@ -434,7 +434,8 @@ int bcfd_block_get_mixed_omega(bcfd_handle h, double* omega);
  * on co-resident CTAs per SM (0 = occupancy limit), and the FP64 solve's
  * phase sync (0 point-to-point between neighbour tiles, 1 grid-wide) */
 int bcfd_block_set_solve_launch(bcfd_handle h, int threads, int ctas_per_sm, int fp64_sync);
-/* out[6] = FP64 solve threads, CTAs/SM cap, sync; FP32 correction threads,
+/* out[6] = FP64 solve threads, CTAs/SM cap, sync (2: the resident solve, each
+ * SM keeping a tile of pc in shared memory); FP32 correction threads,
  * CTAs/SM cap, variant (0 = library default; 1 with 512 threads: the resident
  * sweeps) */
 int bcfd_block_get_solve_launch(bcfd_handle h, int* out);
