@@ -381,6 +381,7 @@ struct Fields4c {
 struct DagArgs {
   int mode;       // 0 or 1
   int vel;        // 1: velocity (6 tasks per IB cell), 0: pressure
+  int keep;       // 1: the dependencies and outputs are read after the call (a recorder)
 };
 
 // latest task before `pos` writing stencil point (a,b,c) of component axis
@@ -413,10 +414,88 @@ __device__ __forceinline__ bool is_last_writer(const DevBlock& B, const DagArgs&
   return B.ibmap[d.idx(a1, b1, c1)] < 0;
 }
 
+// One task per thread (the usual case): probe and dependencies stay in
+// registers, and a task starts as soon as its dependencies' outputs arrive,
+// without a barrier per level.  An output travels as two packets {half of the
+// value, 1} in the task's dependency slot (unused here), so a reader polls the
+// value itself; a lane that is ready never waits for one that is not (a warp
+// loops until all its lanes are done), and all CTAs are co-resident.  A call's
+// time is the FP64 latency of probe and reconstruction along the dependency
+// chain: 73-76 us with a barrier and a new probe per level, 36 us so (1192 and
+// 2131 IB cells).  More tasks than threads, or a recorder, take the levels.
+__device__ __forceinline__ void dag_flow(const DevBlock& B, const DagArgs& g, const DagScratch& s, const GridBar& gb,
+                                         int t, int nt) {
+  ulonglong2* const out = reinterpret_cast<ulonglong2*>(s.dep);
+  const bool mine = t < nt;
+  const int n = g.vel ? t / 6 : t, comp = g.vel ? t % 6 : -1;
+  Probe P;
+  int dep[8];
+  double f[8];
+  unsigned need = 0;
+  if (mine) {
+    __stcg(out + 2 * (int64_t)t, make_ulonglong2(0ull, 0ull));
+    P = make_probe(B, g.mode, comp, n);
+    const double* arr = comp_array(B, P.axis, g.vel != 0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int a = P.ii + (q & 1), b = P.jj + ((q >> 1) & 1), c = P.kk + (q >> 2);
+      dep[q] = last_writer(B, g, P.axis, a, b, c, t);
+      if (dep[q] >= 0) need |= 1u << q;
+      else f[q] = arr[B.d.idx(a, b, c)];
+    }
+  }
+  if (!grid_sync(gb)) return;
+  bool done = !mine;
+  const unsigned long long t0 = globaltimer_ns();
+  for (unsigned spins = 0;; ++spins) {
+    if (!done) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (!(need & (1u << q))) continue;
+        unsigned long long lo, hi;
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                     : "=l"(lo), "=l"(hi)
+                     : "l"(out + 2 * (int64_t)dep[q])
+                     : "memory");
+        if ((lo >> 32) != 1ull || (hi >> 32) != 1ull) continue;
+        f[q] = __hiloint2double((int)hi, (int)lo);
+        need &= ~(1u << q);
+      }
+      if (need == 0) {
+        const double v = reconstruct(B, g.mode, comp, P, f);
+        asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(out + 2 * (int64_t)t),
+                     "l"((1ull << 32) | (unsigned)__double2loint(v)), "l"((1ull << 32) | (unsigned)__double2hiint(v))
+                     : "memory");
+        f[0] = v;
+        done = true;
+      }
+    }
+    if (__all_sync(0xffffffffu, done)) break;
+    if ((spins & 255u) == 255u) {
+      bool stop = (ld_relaxed_u64(gb.ctr) & kBarAbandon) != 0;
+      if (!stop && globaltimer_ns() - t0 > gb.limit_ns) {
+        atomicCAS(gb.err, 0, BCFD_E_TIMEOUT);
+        atomicOr(gb.ctr, kBarAbandon);
+        stop = true;
+      }
+      if (__any_sync(0xffffffffu, stop)) break;
+    }
+  }
+  // every task has read its stencil: the last writers store
+  if (!grid_sync(gb)) return;
+  if (mine && done && is_last_writer(B, g, t, P)) comp_array(B, P.axis, g.vel != 0)[B.d.idx(P.ti, P.tj, P.tk)] = f[0];
+}
+
 __global__ void __launch_bounds__(256) k_forcing_dag(DevBlock B, DagArgs g, DagScratch s, GridBar gb) {
   const int nib = (int)min(B.cnt[C_IB], (int64_t)B.cap_ib);
   const int nt = g.vel ? 6 * nib : nib;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+  // consecutive warps of tasks go to different CTAs: a task is some 250 FP64
+  // instructions, which the FP64 pipe of a few SMs would serialise
+  const int tid = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31), nthr = gridDim.x * blockDim.x;
+  if (!g.keep && nt <= nthr) {
+    dag_flow(B, g, s, gb, tid, nt);
+    return;
+  }
   // phase 1: dependencies
   for (int t = tid; t < nt; t += nthr) {
     const int n = g.vel ? t / 6 : t, comp = g.vel ? t % 6 : -1;
@@ -495,7 +574,7 @@ __global__ void __launch_bounds__(256) k_forcing_dag(DevBlock B, DagArgs g, DagS
 __global__ void k_vel_field(DevBlock B) {
   const int nib = (int)min(B.cnt[C_IB], (int64_t)B.cap_ib);
   const int nt = 6 * nib;
-  const DagArgs g{1, 1};
+  const DagArgs g{1, 1, 0};
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
     const int n = t / 6, comp = t % 6;
     const Probe P = make_probe(B, 1, comp, n);
@@ -786,7 +865,7 @@ static int launch_dag(HostBlock* hb, int mode, int vel) {
   const unsigned grid = coop_grid((const void*)k_forcing_dag, threads, 0, std::min(want, 2u * (unsigned)num_sms()));
   GridBar gb = make_bar(hb->d.err, grid);
   gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
-  DagArgs g{mode, vel};
+  DagArgs g{mode, vel, lib().recorder != nullptr};
   DevBlock B = hb->d;
   void* args[] = {(void*)&B, (void*)&g, (void*)&s, (void*)&gb};
   BCFD_CUDA(launch_coop((const void*)k_forcing_dag, grid, threads, args));
