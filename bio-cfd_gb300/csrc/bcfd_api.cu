@@ -466,6 +466,7 @@ int upload_coefs(HostBlock* hb) {
     hb->d.ca[t] = hb->coef_buf + off[3 + t];
     hb->d.ck[t] = hb->coef_buf + off[3 + N_TAB + t];
   }
+  TRY(launch_diag(hb));
   return hb->ca[0].empty() ? 0 : launch_momentum_tables(hb);
 }
 

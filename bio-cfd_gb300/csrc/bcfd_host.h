@@ -265,6 +265,7 @@ int launch_momentum(const std::vector<HostBlock*>& hbs, double dt, double re, bo
 // fast = 1 (residual-target solves only): the division-free FP64 update
 int launch_sor_set(const std::vector<HostBlock*>& hbs, int64_t itmax, double dt, double epsi, double res_tol,
                    int fast = 0);
+int launch_diag(HostBlock* hb);
 bool tb_solve_fits(HostBlock* hb);
 bool zm_solve_fits(HostBlock* hb);
 bool res_solve_fits(HostBlock* hb);

@@ -123,8 +123,8 @@ struct DevBlock {
   uint8_t* tsnear;  // 1 where a cell is within [-3,3]^3 of a TS cell (overlay stencil)
   // colour-packed Poisson arrays: [0] black, [1] red
   double *pc[2], *rhs[2];
-  // FP64 sweeps (allocated by a block's first FP64 solve): the diagonal
-  // (ax2 + ay2) + az2 of each updated cell and its reciprocal as k_rhs leaves it
+  // the diagonal (ax2 + ay2) + az2 of each interior cell (allocated by a block's
+  // first solve) and its reciprocal as k_rhs leaves it (by its first FP64 solve)
   double *dg[2], *dgi[2];
   float *pcf[2], *rhsf[2];
   uint8_t* upd[2];  // 1 where the packed cell is a fluid cell updated by SOR

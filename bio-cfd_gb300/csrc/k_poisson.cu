@@ -20,6 +20,14 @@ namespace bcfd {
 
 namespace {
 
+// running maximum of magnitudes as bit patterns: non-negative doubles order as
+// integers and a NaN lies above everything, so the result is nmax's, without
+// its two FP64 comparisons (the FP64 pipe is the scarce one)
+__device__ __forceinline__ void bit_max(unsigned long long& m, double x) {
+  m = max(m, (unsigned long long)__double_as_longlong(fabs(x)));
+}
+__device__ __forceinline__ double bit_value(unsigned long long m) { return __longlong_as_double((long long)m); }
+
 // computeDiv (src/PcorVcor.F90:222-243) over the fluid cells; b lands in the
 // packed layout.  Non-fluid cells keep the zero of the start of the solve.
 // With `fast` (the residual-target solves, which reproduce no reference bits)
@@ -69,20 +77,10 @@ __device__ __forceinline__ double div_by(double v, double d, double s) {
   return q;
 }
 
-// What the FP64 sweeps of one solve read beside pc, per updated cell:
-//  * rhs = b / deltat (the reference divides inside every sweep; the quotient
-//    is the same IEEE value);
-//  * dg = (ax2 + ay2) + az2, the diagonal, in the reference's order;
-//  * dgi: with `fast`, omega times the reciprocal of the diagonal (an FP32
-//    reciprocal refined by one Newton-Raphson step, y1 = y0 + y0 (1 - d y0));
-//    else the correctly rounded reciprocal y = 1/dg that div_by takes, stored
-//    with its sign cleared where div_by needs its second correction and as
-//    NaN where dg is out of the range its proof covers.
-// One pass per solve (one division per cell) replaces an addition pair and a
-// division in every one of the solve's hundreds of updates per cell: GB300
-// issues FP64 at 1/64 of the FP32 rate, so the FP64 sweeps are bound by their
-// count of FP64 instructions (memory is at 10-15% of its rate).
-__global__ void k_rhs(DevBlock B, double dt, double omega, int fast) {
+// dg = (ax2 + ay2) + az2, the diagonal in the reference's order, at every
+// interior cell (0 elsewhere): made when the line tables change, read by the
+// FP64 sweeps and the residual passes instead of two FP64 additions per cell
+__global__ void k_diag(DevBlock B) {
   const Dims& d = B.d;
   const int64_t n = d.npacked();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
@@ -92,10 +90,34 @@ __global__ void k_rhs(DevBlock B, double dt, double omega, int fast) {
     const int j = 1 + (int)(r % d.NY), k = 1 + (int)(r / d.NY);
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
+      const int i = 2 * h + 1 + (((1 + j + k) & 1) != c);
+      const bool in = i >= 2 && i <= d.nx + 1 && j >= 2 && j <= d.ny + 1 && k >= 2 && k <= d.nz + 1;
+      B.dg[c][t] = in ? B.Acx[i - 2 + d.nx] + B.Acy[j - 2 + d.ny] + B.Acz[k - 2 + d.nz] : 0.0;
+    }
+  }
+}
+
+// What the FP64 sweeps of one solve read beside pc, per updated cell:
+//  * rhs = b / deltat (the reference divides inside every sweep; the quotient
+//    is the same IEEE value);
+//  * dgi: from the diagonal dg (k_diag), with `fast`, omega times the reciprocal of the diagonal (an FP32
+//    reciprocal refined by one Newton-Raphson step, y1 = y0 + y0 (1 - d y0));
+//    else the correctly rounded reciprocal y = 1/dg that div_by takes, stored
+//    with its sign cleared where div_by needs its second correction and as
+//    NaN where dg is out of the range its proof covers.
+// One pass per solve (one division per cell) replaces an addition pair and a
+// division in every one of the solve's hundreds of updates per cell: GB300
+// issues FP64 at 1/64 of the FP32 rate, so the FP64 sweeps are bound by their
+// count of FP64 instructions (memory is at 10-15% of its rate).
+__global__ void k_rhs(DevBlock B, double dt, double omega, int fast) {
+  const int64_t n = B.d.npacked();
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
+       t += (int64_t)gridDim.x * blockDim.x) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
       B.rhs[c][t] = B.bpk[c][t] / dt;
       if (!B.upd[c][t]) continue;
-      const int i = 2 * h + 1 + (((1 + j + k) & 1) != c);
-      const double dg = B.Acx[i - 2 + d.nx] + B.Acy[j - 2 + d.ny] + B.Acz[k - 2 + d.nz];
+      const double dg = B.dg[c][t];
       double y;
       if (fast) {
         const double y0 = (double)__frcp_rn((float)dg);
@@ -106,7 +128,6 @@ __global__ void k_rhs(DevBlock B, double dt, double omega, int fast) {
       } else {
         y = __longlong_as_double(0x7ff8000000000000ll);
       }
-      B.dg[c][t] = dg;
       B.dgi[c][t] = y;
     }
   }
@@ -312,7 +333,7 @@ __device__ __forceinline__ void tile_half64(const DevBlock& B, const Tile& t, do
       }
       if (u == 0 ? mk.x : mk.y) {
         nv[u] = v;
-        if (CHK) lmax = max(lmax, (unsigned long long)__double_as_longlong(fabs(v - old)));
+        if (CHK) bit_max(lmax, v - old);
       }
     }
     // cells that are not updated keep their value; no other CTA writes them
@@ -346,15 +367,15 @@ __device__ __forceinline__ double resid64_cell(const DevBlock& B, const Pos& p) 
 // of the FP64 residual-target solve)
 template <int C>
 __device__ __forceinline__ double tile_resid_max64(const DevBlock& B, const Tile& t) {
-  double m = 0.0;
+  unsigned long long m = 0;
   const int n = B.d.NXH * t.nj * t.nk;
   Walk3 w;
   w.init(threadIdx.x, blockDim.x, B.d.NXH, t.nj);
   for (int q = threadIdx.x; q < n; q += blockDim.x, w.next()) {
     const Pos p = tile_pos<C>(B, t, w, true);
-    if (p.on) m = nmax(m, fabs(resid64_cell<C>(B, p)));
+    if (p.on) bit_max(m, resid64_cell<C>(B, p));
   }
-  return m;
+  return bit_value(m);
 }
 
 // max over fluid cells of colour C of |b/dt - A pc| (grid-stride; measurement)
@@ -364,7 +385,7 @@ __device__ __forceinline__ double resid_max64(const DevBlock& B, int64_t total) 
   const double* own = B.pc[C];
   const double* o = B.pc[1 - C];
   const int64_t sy = d.NXH, sz = (int64_t)d.NXH * d.NY;
-  double m = 0.0;
+  unsigned long long m = 0;
   const int S = gridDim.x * blockDim.x;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   Walk3 w;
@@ -383,9 +404,9 @@ __device__ __forceinline__ double resid_max64(const DevBlock& B, int64_t total) 
     ax = fma(B.Acy[j - 2 + 2 * d.ny], __ldcg(o + pi + sy), ax);
     ax = fma(B.Acz[k - 2], __ldcg(o + pi - sz), ax);
     ax = fma(B.Acz[k - 2 + 2 * d.nz], __ldcg(o + pi + sz), ax);
-    m = nmax(m, fabs(B.rhs[C][pi] - ax));
+    bit_max(m, B.rhs[C][pi] - ax);
   }
-  return m;
+  return bit_value(m);
 }
 
 struct SorArgs {
@@ -489,7 +510,7 @@ __device__ __forceinline__ void sor64_body(const DevBlock& B, const SorArgs& a, 
     sor64_half<0>(B, t, a, !target_mode && r5 == 0, lbits);
     tile_publish(tm, t, ++ph);
     if (target_mode ? it >= next_check : r5 == 0) {
-      double lmax = __longlong_as_double((long long)lbits);
+      double lmax = bit_value(lbits);
       if (target_mode) {
         // residual-target mode: the residual needs the neighbours' sweep pair
         if (!tile_wait(tm, gb, t, ph)) { ok = false; break; }
@@ -568,6 +589,36 @@ __device__ __forceinline__ int next_inner(const DcArgs& a, int outer, double res
   return min(a.inner, max(kMinInner, (int)ceil(need * 1.15) + 2));
 }
 
+// L2 policies of the FP32 sweeps' accesses.  A half-sweep reads half of e, half
+// of the right-hand side and writes half of e; on a block beyond L2 everything
+// came from DRAM in turn.  The right-hand side, read once per pair, is marked
+// to go first, and half of e to stay, so that part of e is found in L2 by the
+// next half-sweeps (384x256x256: 77.1 -> 69.9 us per pair; all of e marked to
+// stay 71.8, no part of it 73.2; blocks whose e and right-hand side fit L2 are
+// within 2% either way)
+__device__ __forceinline__ uint64_t l2_policy_keep() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, 0.5;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint64_t l2_policy_stream() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ float4 ld4(const float* a, uint64_t pol) {
+  float4 v;
+  asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(a), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ void st4(float* a, const float4& v, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(a), "f"(v.x), "f"(v.y), "f"(v.z),
+               "f"(v.w), "l"(pol)
+               : "memory");
+}
+
 // one FP32 half-sweep of colour C over the tile.  Each thread updates a run
 // of four consecutive packed cells h0..h0+3 of one row (h0 a multiple of 4;
 // rows are 16-byte aligned): the run shares one x-parity `par` (its cells sit
@@ -577,7 +628,8 @@ __device__ __forceinline__ int next_inner(const DcArgs& a, int outer, double res
 // run is written back with one float4 store (cells that are not updated keep
 // their value; no other CTA writes them in this phase).
 template <int C>
-__device__ __forceinline__ void tile_half32(const DevBlock& B, const Tile& t, float omega) {
+__device__ __forceinline__ void tile_half32(const DevBlock& B, const Tile& t, float omega, uint64_t keep,
+                                            uint64_t strm) {
   const Dims& d = B.d;
   const float* __restrict__ o = B.pcf[1 - C];
   float* __restrict__ own = B.pcf[C];
@@ -596,13 +648,13 @@ __device__ __forceinline__ void tile_half32(const DevBlock& B, const Tile& t, fl
     // exit on the mask: all addresses of a tile row are in range)
     const uchar4 m = *reinterpret_cast<const uchar4*>(upd + pi);
     const int par = ((1 + j + k) & 1) != C;
-    const float4 oc = *reinterpret_cast<const float4*>(o + pi);
-    const float4 os = *reinterpret_cast<const float4*>(o + pi - sy);
-    const float4 on = *reinterpret_cast<const float4*>(o + pi + sy);
-    const float4 ob = *reinterpret_cast<const float4*>(o + pi - sz);
-    const float4 ot = *reinterpret_cast<const float4*>(o + pi + sz);
-    const float4 r4 = *reinterpret_cast<const float4*>(rhs + pi);
-    const float4 e4 = *reinterpret_cast<const float4*>(own + pi);
+    const float4 oc = ld4(o + pi, keep);
+    const float4 os = ld4(o + pi - sy, keep);
+    const float4 on = ld4(o + pi + sy, keep);
+    const float4 ob = ld4(o + pi - sz, keep);
+    const float4 ot = ld4(o + pi + sz, keep);
+    const float4 r4 = ld4(rhs + pi, strm);
+    const float4 e4 = ld4(own + pi, keep);
     // the one x-neighbour outside the centre float4 (in range: row +- 1)
     const float ox = par ? o[pi + 4] : o[pi - 1];
     const float4 cy = B.ayr[j - 2], cz = B.azr[k - 2];
@@ -638,8 +690,29 @@ __device__ __forceinline__ void tile_half32(const DevBlock& B, const Tile& t, fl
       const float nvv = __fmaf_rn(omega, __fdividef(s, ax2 + ay2 + az2) - ev[u], ev[u]);
       ev[u] = mv[u] ? nvv : ev[u];
     }
-    *reinterpret_cast<float4*>(own + pi) = make_float4(ev[0], ev[1], ev[2], ev[3]);
+    st4(own + pi, make_float4(ev[0], ev[1], ev[2], ev[3]), keep);
   }
+}
+
+// (float)x by integer arithmetic (round to nearest even): GB300 converts in the
+// FP64 pipe, which bounds the residual pass; zeros, and exponents outside
+// FP32's normal range by the conversion
+__device__ __forceinline__ float to_f32(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned e = (hi >> 20) & 0x7ffu;
+  unsigned f = ((hi & 0x7fffffffu) << 3 | lo >> 29) - (896u << 23);
+  const unsigned rem = lo & 0x1fffffffu;
+  f += (rem > 0x10000000u || (rem == 0x10000000u && (f & 1u))) ? 1u : 0u;
+  float r = __uint_as_float((hi & 0x80000000u) | f);
+  if (e - 897u >= 254u) r = (float)x;
+  return r;
+}
+// (double)x of a normal number or zero by integer arithmetic (exact)
+__device__ __forceinline__ double to_f64(float x) {
+  const unsigned u = __float_as_uint(x), e = (u >> 23) & 0xffu;
+  double r = __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+  if (e - 1u >= 254u) r = (double)x;
+  return r;
 }
 
 // FP64 residual r = b * (1/dt) - A pc of colour C over the tile, two
@@ -660,7 +733,7 @@ __device__ __forceinline__ double tile_residual64v(const DevBlock& B, const Tile
   const int nh = d.NXH >> 1;
   const int64_t sy = d.NXH, sz = (int64_t)d.NXH * d.NY;
   const int n = nh * t.nj * t.nk;
-  double m = 0.0;
+  unsigned long long m = 0;
   Walk3 w;
   w.init(threadIdx.x, blockDim.x, nh, t.nj);
   for (int q = threadIdx.x; q < n; q += blockDim.x, w.next()) {
@@ -676,16 +749,17 @@ __device__ __forceinline__ double tile_residual64v(const DevBlock& B, const Tile
     const double2 x2 = *reinterpret_cast<const double2*>(x + pi);
     const double2 b2 = *reinterpret_cast<const double2*>(bb + pi);
     const double ox = par ? o[pi + 2] : o[pi - 1];
-    const double ay1 = B.Acy[j - 2], ay2 = B.Acy[j - 2 + d.ny], ay3 = B.Acy[j - 2 + 2 * d.ny];
-    const double az1 = B.Acz[k - 2], az2 = B.Acz[k - 2 + d.nz], az3 = B.Acz[k - 2 + 2 * d.nz];
+    const double2 d2 = *reinterpret_cast<const double2*>(B.dg[C] + pi);
+    const double ay1 = B.Acy[j - 2], ay3 = B.Acy[j - 2 + 2 * d.ny];
+    const double az1 = B.Acz[k - 2], az3 = B.Acz[k - 2 + 2 * d.nz];
     double r[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const double left = u == 0 ? (par ? oc.x : ox) : (par ? oc.y : oc.x);
       const double right = u == 0 ? (par ? oc.y : oc.x) : (par ? ox : oc.y);
       const int ic = min(max(2 * (h0 + u) + 1 + par, 2), d.nx + 1);
-      const double ax1 = B.Acx[ic - 2], ax2 = B.Acx[ic - 2 + d.nx], ax3 = B.Acx[ic - 2 + 2 * d.nx];
-      double ax = (ax2 + ay2 + az2) * (u == 0 ? x2.x : x2.y);
+      const double ax1 = B.Acx[ic - 2], ax3 = B.Acx[ic - 2 + 2 * d.nx];
+      double ax = (u == 0 ? d2.x : d2.y) * (u == 0 ? x2.x : x2.y);
       ax = fma(ax1, left, ax);
       ax = fma(ax3, right, ax);
       ax = fma(ay1, u == 0 ? os.x : os.y, ax);
@@ -694,11 +768,11 @@ __device__ __forceinline__ double tile_residual64v(const DevBlock& B, const Tile
       ax = fma(az3, u == 0 ? ot.x : ot.y, ax);
       r[u] = (u == 0 ? b2.x : b2.y) * inv_dt - ax;
     }
-    if (mk.x) m = nmax(m, fabs(r[0]));
-    if (mk.y) m = nmax(m, fabs(r[1]));
-    *reinterpret_cast<float2*>(rf + pi) = make_float2(mk.x ? (float)r[0] : 0.0f, mk.y ? (float)r[1] : 0.0f);
+    if (mk.x) bit_max(m, r[0]);
+    if (mk.y) bit_max(m, r[1]);
+    *reinterpret_cast<float2*>(rf + pi) = make_float2(mk.x ? to_f32(r[0]) : 0.0f, mk.y ? to_f32(r[1]) : 0.0f);
   }
-  return m;
+  return bit_value(m);
 }
 
 // x += e in FP64 over the tile's updated cells of colour C, e back to 0; runs
@@ -720,10 +794,10 @@ __device__ __forceinline__ void tile_apply4(const DevBlock& B, const Tile& t) {
     const float4 e4 = *reinterpret_cast<const float4*>(e + pi);
     double2 a = *reinterpret_cast<const double2*>(x + pi);
     double2 b = *reinterpret_cast<const double2*>(x + pi + 2);
-    if (mk.x) a.x = a.x + (double)e4.x;
-    if (mk.y) a.y = a.y + (double)e4.y;
-    if (mk.z) b.x = b.x + (double)e4.z;
-    if (mk.w) b.y = b.y + (double)e4.w;
+    if (mk.x) a.x = a.x + to_f64(e4.x);
+    if (mk.y) a.y = a.y + to_f64(e4.y);
+    if (mk.z) b.x = b.x + to_f64(e4.z);
+    if (mk.w) b.y = b.y + to_f64(e4.w);
     *reinterpret_cast<double2*>(x + pi) = a;
     *reinterpret_cast<double2*>(x + pi + 2) = b;
     *reinterpret_cast<float4*>(e + pi) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -736,6 +810,7 @@ __device__ __forceinline__ void sor_dc_body(const DevBlock& B, const DcArgs& a, 
   const Tile t = my_tile(B.d, tm, cta);
   BlockStats* st = B.stats;
   int64_t sweeps = 0;
+  const uint64_t keep = l2_policy_keep(), strm = l2_policy_stream();
   double res = 0.0, res_prev = 0.0;
   int inner = a.inner;
   unsigned ph = 0;
@@ -753,10 +828,10 @@ __device__ __forceinline__ void sor_dc_body(const DevBlock& B, const DcArgs& a, 
     res_prev = res;
     for (int it = 0; it < inner; ++it) {
       if (!tile_wait(tm, gb, t, ph)) return;
-      tile_half32<1>(B, t, a.omega);
+      tile_half32<1>(B, t, a.omega, keep, strm);
       tile_publish(tm, t, ++ph);
       if (!tile_wait(tm, gb, t, ph)) return;
-      tile_half32<0>(B, t, a.omega);
+      tile_half32<0>(B, t, a.omega, keep, strm);
       tile_publish(tm, t, ++ph);
     }
     sweeps += inner;
@@ -1663,10 +1738,10 @@ __device__ __forceinline__ void res_apply(const DevBlock& B, const ResTile& R) {
         (C ? R.er + R.red(w.b, w.c) * R.nxh : R.eb + R.black(w.b, w.c) * R.nxh) + 4 * w.a);
     double2 a = *reinterpret_cast<const double2*>(x + pi);
     double2 b = *reinterpret_cast<const double2*>(x + pi + 2);
-    if (m & 1u) a.x = a.x + (double)e4.x;
-    if (m & 2u) a.y = a.y + (double)e4.y;
-    if (m & 4u) b.x = b.x + (double)e4.z;
-    if (m & 8u) b.y = b.y + (double)e4.w;
+    if (m & 1u) a.x = a.x + to_f64(e4.x);
+    if (m & 2u) a.y = a.y + to_f64(e4.y);
+    if (m & 4u) b.x = b.x + to_f64(e4.z);
+    if (m & 8u) b.y = b.y + to_f64(e4.w);
     *reinterpret_cast<double2*>(x + pi) = a;
     *reinterpret_cast<double2*>(x + pi + 2) = b;
   }
@@ -2007,7 +2082,7 @@ __device__ __forceinline__ void res64_rows(const DevBlock& B, const Res64Args& z
           ax = fma(az1, pb, ax);
           ax = fma(az3, pt, ax);
           v = v - ax;
-          if (u == 0 ? mk.x : mk.y) lmax = max(lmax, (unsigned long long)__double_as_longlong(fabs(v)));
+          if (u == 0 ? mk.x : mk.y) bit_max(lmax, v);
           continue;
         }
         if (WHAT == 1) {
@@ -2025,7 +2100,7 @@ __device__ __forceinline__ void res64_rows(const DevBlock& B, const Res64Args& z
         }
         if (u == 0 ? mk.x : mk.y) {
           nv[u] = v;
-          if (chk) lmax = max(lmax, (unsigned long long)__double_as_longlong(fabs(v - old)));
+          if (chk) bit_max(lmax, v - old);
         }
       }
     }
@@ -2170,9 +2245,9 @@ __global__ void __launch_bounds__(kRes64Threads, 1) k_sor64_res(DevBlock B, SorA
             else res64_rows<0, 0, 2>(B, z, R, list, 0, n, pa, slot, 0, 0.0, false, lbits);
           }
         }
-        lmax = __longlong_as_double((long long)lbits) * a.dt;
+        lmax = bit_value(lbits) * a.dt;
       } else {
-        lmax = __longlong_as_double((long long)lbits);
+        lmax = bit_value(lbits);
       }
       const double m = block_max(lmax, sh);
       if (threadIdx.x == 0) atomic_max_nonneg(&st->slot[check % 3], m);
@@ -2324,16 +2399,15 @@ struct SteadyOp {
     __shared__ double sh[32];
     // max |x| / dt = (max |x|) / dt exactly: a correctly rounded division by
     // dt > 0 is monotone, so one division per CTA gives the per-cell result
-    double m = 0.0;
+    unsigned long long mb = 0;
     FOR_INTERIOR(B, cta, ncta) {
       INTERIOR_CELL(B);
       if (B.cell[c] != 0) continue;
-      const double eu = fabs((B.ut[c] - B.u[c]));
-      const double ev = fabs((B.vt[c] - B.v[c]));
-      const double ew = fabs((B.wt[c] - B.w[c]));
-      m = nmax(nmax(nmax(m, eu), ev), ew);
+      bit_max(mb, B.ut[c] - B.u[c]);
+      bit_max(mb, B.vt[c] - B.v[c]);
+      bit_max(mb, B.wt[c] - B.w[c]);
     }
-    m = block_max(m, sh);
+    const double m = block_max(bit_value(mb), sh);
     if (threadIdx.x == 0) atomic_max_nonneg(&B.stats->derr_std_st, m / dt);
   }
 };
@@ -2354,15 +2428,15 @@ struct MaxDivOp {
     const double* rx = B.lcoef + (d.NX + d.NY + d.NZ);
     const double* ry = rx + d.NX;
     const double* rz = ry + d.NY;
-    double m = 0.0;
+    unsigned long long mb = 0;
     FOR_INTERIOR(B, cta, ncta) {
       INTERIOR_CELL(B);
       if (B.cell[c] != 0) continue;
       const double dv = (U[c] - U[c - 1]) * rx[i - 1] + (V[c] - V[c - d.NX]) * ry[j - 1] +
                         (W[c] - W[c - (int64_t)d.NX * d.NY]) * rz[k - 1];
-      m = nmax(m, fabs(dv));
+      bit_max(mb, dv);
     }
-    m = block_max(m, sh);
+    const double m = block_max(bit_value(mb), sh);
     if (threadIdx.x == 0) atomic_max_nonneg(tfield ? &B.stats->pad[0] : &B.stats->maxdiv, m);
   }
 };
@@ -2527,25 +2601,39 @@ static int reset_solve_state(HostBlock* hb, const TileMap& tm) {
   return 0;
 }
 
-// the FP64 sweeps' diagonal arrays (the first FP64 solve of a block)
-static int ensure_diag(HostBlock* hb) {
-  if (hb->d.dg[0]) return 0;
+// two packed FP64 arrays, zeroed (cells that are not updated are read, two per
+// thread, but not used)
+static int ensure_packed_pair(HostBlock* hb, double* (&a)[2]) {
+  if (a[0]) return 0;
   const size_t np = (size_t)hb->d.d.npacked();
   void* p = nullptr;
-  if (cudaMalloc(&p, 4 * np * sizeof(double)) != cudaSuccess) return BCFD_E_NOMEM;
+  if (cudaMalloc(&p, 2 * np * sizeof(double)) != cudaSuccess) return BCFD_E_NOMEM;
   hb->allocs.push_back(p);
-  // cells that are not updated are read (two cells per thread) but not used
-  BCFD_CUDA(cudaMemsetAsync(p, 0, 4 * np * sizeof(double), stream()));
-  double* q = static_cast<double*>(p);
-  for (int c = 0; c < 2; ++c) {
-    hb->d.dg[c] = q + c * np;
-    hb->d.dgi[c] = q + (2 + c) * np;
-  }
+  BCFD_CUDA(cudaMemsetAsync(p, 0, 2 * np * sizeof(double), stream()));
+  a[0] = static_cast<double*>(p);
+  a[1] = a[0] + np;
   return 0;
+}
+
+// the block's diagonal from its current line tables, if it has been used
+int launch_diag(HostBlock* hb) {
+  if (!hb->d.dg[0]) return 0;
+  k_diag<<<grid_for(hb->d.d.npacked(), 256), 256, 0, stream()>>>(hb->d);
+  BCFD_LAUNCHED();
+  return 0;
+}
+
+// the diagonal (the first solve of a block makes it, later changes of the line
+// tables remake it; the transposed tables of the adjoint have the same one)
+static int ensure_diag(HostBlock* hb) {
+  if (hb->d.dg[0]) return 0;
+  TRY_R(ensure_packed_pair(hb, hb->d.dg));
+  return launch_diag(hb);
 }
 
 static int launch_rhs(HostBlock* hb, double dt, int fast) {
   TRY_R(ensure_diag(hb));
+  TRY_R(ensure_packed_pair(hb, hb->d.dgi));
   k_rhs<<<grid_for(hb->d.d.npacked(), 256), 256, 0, stream()>>>(hb->d, dt, hb->omega, fast);
   BCFD_LAUNCHED();
   return 0;
@@ -2927,6 +3015,7 @@ static int launch_sor_res(HostBlock* hb, int64_t itmax, double dt, double div_to
 int launch_sor_mixed(HostBlock* hb, int64_t itmax, double dt, double div_tol) {
   DevBlock& B = hb->d;
   const int64_t np = B.d.npacked();
+  TRY_R(ensure_diag(hb));
   // the resident sweeps by choice, or by default (no launch shape asked for)
   // wherever they fit: on every such size measured they are faster than the
   // tiled ones, 4.64 -> 1.47 us per sweep pair on 33x21x27, 5.2 -> 2.4 on 64^3,
@@ -3046,6 +3135,7 @@ int launch_sor_mixed_set(const std::vector<HostBlock*>& hbs, int64_t itmax, doub
   }
   const int threads = kDcThreads;
   for (HostBlock* hb : hbs) {
+    TRY_R(ensure_diag(hb));
     if (hb->dc_variant >= 2 || hb->dc_threads > 0 || hb->dc_ctas_per_sm > 0) continue;
     for (int c = 0; c < 2; ++c)
       BCFD_CUDA(cudaMemsetAsync(hb->d.pcf[c], 0, hb->d.d.npacked() * sizeof(float), stream()));
