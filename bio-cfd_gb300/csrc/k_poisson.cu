@@ -258,10 +258,11 @@ __device__ __forceinline__ Pos tile_pos(const DevBlock& B, const Tile& t, const 
   return p;
 }
 
-// (bound by the FP64 pipe: 20-23 FP64 instructions per update against 29 with
-// the division and the diagonal's sum in every update, 8 against 17 with FAST;
-// 384x256x256: 2063 -> 1017 us per sweep pair, FAST 920 -> 389 us; 128x96x96:
-// 108 -> 58 and 52 -> 25 us)
+// pairs of packed cells of a row that can hold an interior cell (the last one
+// is h = nx / 2); the row's padding costs FP64 instructions like any cell, so
+// the loops leave it out (two-block sphere run in FP64: 73.2 -> 66.9 ms)
+__device__ __forceinline__ int row_pairs(const Dims& d) { return (d.nx >> 2) + 1; }
+
 // One FP64 half-sweep of colour C over the tile, two consecutive packed cells
 // per thread (double2 loads as in tile_residual64v).  FAST = 0: the
 // reference's update (no FMA, the expression order of src/PcorVcor.F90:319-327,
@@ -272,6 +273,10 @@ __device__ __forceinline__ Pos tile_pos(const DevBlock& B, const Tile& t, const 
 // max |new - old| as a bit pattern (of non-negative numbers: ordered as
 // integers, NaN above everything), needed only by the half-sweeps before the
 // reference's stop test.
+// (bound by the FP64 pipe: 20-23 FP64 instructions per update against 29 with
+// the division and the diagonal's sum in every update, 8 against 17 with FAST;
+// 384x256x256: 2063 -> 1017 us per sweep pair, FAST 920 -> 389 us; 128x96x96:
+// 108 -> 58 and 52 -> 25 us)
 template <int C, int FAST, int CHK>
 __device__ __forceinline__ void tile_half64(const DevBlock& B, const Tile& t, double omega,
                                             unsigned long long& lmax) {
@@ -282,7 +287,7 @@ __device__ __forceinline__ void tile_half64(const DevBlock& B, const Tile& t, do
   const double* __restrict__ dgp = B.dg[C];
   const double* __restrict__ dip = B.dgi[C];
   const uint8_t* __restrict__ upd = B.upd[C];
-  const int nh = d.NXH >> 1, nx = d.nx, ny = d.ny, nz = d.nz;
+  const int nh = row_pairs(d), nx = d.nx, ny = d.ny, nz = d.nz;
   const int64_t sy = d.NXH, sz = (int64_t)d.NXH * d.NY;
   const int n = nh * t.nj * t.nk;
   const double om1 = 1.0 - omega;
@@ -730,7 +735,7 @@ __device__ __forceinline__ double tile_residual64v(const DevBlock& B, const Tile
   const double* __restrict__ bb = B.bpk[C];
   const uint8_t* __restrict__ upd = B.upd[C];
   float* __restrict__ rf = B.rhsf[C];
-  const int nh = d.NXH >> 1;
+  const int nh = row_pairs(d);
   const int64_t sy = d.NXH, sz = (int64_t)d.NXH * d.NY;
   const int n = nh * t.nj * t.nk;
   unsigned long long m = 0;
@@ -2037,7 +2042,7 @@ template <int C, int PAR, int WHAT>
 __device__ __forceinline__ void res64_rows(const DevBlock& B, const Res64Args& z, const Res64Tile& R,
                                            const unsigned short* list, int nedge, int n, int a, int slot, unsigned ph,
                                            double omega, bool chk, unsigned long long& lmax) {
-  const int nxh = R.nxh, nj = R.t.nj, nk = R.t.nk, nx = B.d.nx;
+  const int nxh = R.nxh, nj = R.t.nj, nx = B.d.nx;
   const double* __restrict__ o = R.e[1 - C] + 2 * a;
   double* __restrict__ own = R.e[C] + 2 * a;
   const int sk = (nj + 2) * nxh;
