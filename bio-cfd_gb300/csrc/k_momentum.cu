@@ -721,12 +721,21 @@ struct MomentumTsOp {
     __shared__ int s_last[NT][N_KIND], s_list[NT], s_n;
     const Dims& d = B.d;
     const int nts = (int)min(B.cnt[C_TS], (int64_t)B.cap_ib);
+    if (nts == 0) return;  // no cell is near one
     const int64_t n = (int64_t)d.nx * d.ny * d.nz;
+    // 32-bit divisions when the interior count fits them
     auto cell_at = [&](int64_t t, int& i, int& j, int& k) {
-      i = 2 + (int)(t % d.nx);
-      const int64_t r = t / d.nx;
-      j = 2 + (int)(r % d.ny);
-      k = 2 + (int)(r / d.ny);
+      if (n <= 0x7fffffffLL) {
+        const unsigned r = (unsigned)t / (unsigned)d.nx;
+        i = 2 + (int)((unsigned)t - r * (unsigned)d.nx);
+        k = 2 + (int)(r / (unsigned)d.ny);
+        j = 2 + (int)(r - (unsigned)(k - 2) * (unsigned)d.ny);
+      } else {
+        i = 2 + (int)(t % d.nx);
+        const int64_t r = t / d.nx;
+        j = 2 + (int)(r % d.ny);
+        k = 2 + (int)(r / d.ny);
+      }
     };
     for (int64_t t0 = (int64_t)cta * NT; t0 < n; t0 += (int64_t)ncta * NT) {
       const int64_t t = t0 + threadIdx.x;
