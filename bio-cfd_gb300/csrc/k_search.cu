@@ -105,6 +105,9 @@ __device__ void warp_nearest(const QueryCtx& C, const double (&q)[Q][3], int (&o
     mf[s] = kFInf;
   }
   // one chunk: every query's minimum over its elements (warp-uniform result)
+  // by one reduction of the bit patterns (distances are not negative: ordered
+  // as integers, NaN above all) instead of five exchanges per query and chunk,
+  // the chain that bounds a query: moved 160x144x96 plate 2.55 -> 2.45 ms
   auto visit1 = [&](int c) {
     const int pos = 32 * c + lane;
     float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -113,8 +116,8 @@ __device__ void warp_nearest(const QueryCtx& C, const double (&q)[Q][3], int (&o
 #pragma unroll
     for (int s = 0; s < Q; ++s) {
       float v = in ? fdist2(qf[s][0] - e.x, qf[s][1] - e.y, qf[s][2] - e.z) : kFInf;
-      for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-      mf[s] = fminf(mf[s], v);
+      v = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(fminf(v, mf[s]))));
+      mf[s] = v;
     }
   };
 #pragma unroll
