@@ -174,18 +174,24 @@ __device__ __forceinline__ Dual4 operator*(const Dual4& a, const Dual4& b) {
 }
 __device__ __forceinline__ Dual4 fabs(const Dual4& a) { return a.v < 0.0 ? -a : a; }
 
-// grid quantities have no tangent: plain numbers beside the dual types (the
-// tangent's zero products left out)
-template <typename T>
+// Grid quantities have no tangent: plain numbers beside the dual types, the
+// tangent's products with their zeros left out.  Those products are zeros only
+// while the values are finite; an infinite or NaN value makes the tangent of
+// everything that it enters NaN, and a derivative taken at such a state must
+// not look like a number.  EXACT keeps them: the grid quantities are dual
+// numbers with tangent 0, with the operations of a dual quotient.  Every value
+// that enters an output makes that output non-finite when it is not finite
+// itself, so finite outputs tell that the short form gives EXACT's bits.
+template <typename T, bool EXACT>
 struct GridNum {
   using type = T;
 };
 template <>
-struct GridNum<Dual> {
+struct GridNum<Dual, false> {
   using type = double;
 };
 template <>
-struct GridNum<Dual4> {
+struct GridNum<Dual4, false> {
   using type = double;
 };
 __device__ __forceinline__ Dual operator*(double c, Dual a) { return Dual(c * a.v, c * a.d); }
@@ -202,7 +208,7 @@ __device__ __forceinline__ Dual4 operator*(double c, const Dual4& a) {
 }
 
 // One axis's tables at one grid index.
-template <typename T>
+template <typename T, bool EXACT>
 struct MomAxis {
   static constexpr int n = 32;  // entries between slots
   const double* t;
@@ -211,7 +217,7 @@ struct MomAxis {
   __device__ __forceinline__ MomAxis(const DevBlock& B, int g0, int q)
       : t(B.mt + mom_slot0(g0, q - 1, kMtSlots)), f(B.mtf + mom_slot0(g0, q - 1, kMfSlots)),
         k(B.mtk[32 * g0 + q - 1]) {}
-  using G = typename GridNum<T>::type;
+  using G = typename GridNum<T, EXACT>::type;
   // numerator / divisor s: FP64 by div_any (the division's bits); FP32 of the
   // mixed path by the reciprocal (the bits of __fdividef)
   // (V: T, or double where a static seed leaves the operand no tangent)
@@ -226,11 +232,12 @@ struct MomAxis {
       if constexpr (std::is_same<V, double>::value) {
         return div_any(a, d, y, k, s);
       } else if constexpr (std::is_same<V, Dual>::value) {
-        return Dual(div_any(a.v, d, y, k, s), div_any(a.d, d, y, k, s));
+        const double q = div_any(a.v, d, y, k, s);
+        return Dual(q, div_any(EXACT ? a.d - q * 0.0 : a.d, d, y, k, s));
       } else {
         Dual4 r(div_any(a.v, d, y, k, s));
 #pragma unroll
-        for (int l = 0; l < 4; ++l) r.d[l] = div_any(a.d[l], d, y, k, s);
+        for (int l = 0; l < 4; ++l) r.d[l] = div_any(EXACT ? a.d[l] - r.v * 0.0 : a.d[l], d, y, k, s);
         return r;
       }
     }
@@ -238,31 +245,36 @@ struct MomAxis {
   __device__ __forceinline__ G quot(int s) const {
     if constexpr (std::is_same<T, FastF>::value) return G(f[(kMfQ + s) * n]);
     else if constexpr (std::is_same<T, float>::value) return f[(kMfI + s) * n];
-    else return t[(kMtQ + s) * n];
+    else return G(t[(kMtQ + s) * n]);
   }
   // column c (1..5) of CA (kind 0) / CK (1) self, CA (2) / CK (3) cross
   __device__ __forceinline__ G coef(int kind, int c) const {
     if constexpr (std::is_same<T, FastF>::value || std::is_same<T, float>::value)
       return G(f[(kMfC + 5 * kind + c - 1) * n]);
-    else return t[(kMtC + 5 * kind + c - 1) * n];
+    else return G(t[(kMtC + 5 * kind + c - 1) * n]);
   }
 };
 
 // division by re
-template <typename T>
+template <bool EXACT, typename T>
 __device__ __forceinline__ T div_re(const T& a, const MomArgs& m) {
   if constexpr (std::is_same<T, double>::value) {
     return div_any(a, m.re, m.re_y, m.re_k, 0);
   } else if constexpr (std::is_same<T, Dual>::value) {
-    return Dual(div_any(a.v, m.re, m.re_y, m.re_k, 0), div_any(a.d, m.re, m.re_y, m.re_k, 0));
+    const double q = div_any(a.v, m.re, m.re_y, m.re_k, 0);
+    return Dual(q, div_any(EXACT ? a.d - q * 0.0 : a.d, m.re, m.re_y, m.re_k, 0));
   } else if constexpr (std::is_same<T, Dual4>::value) {
     Dual4 r(div_any(a.v, m.re, m.re_y, m.re_k, 0));
 #pragma unroll
-    for (int l = 0; l < 4; ++l) r.d[l] = div_any(a.d[l], m.re, m.re_y, m.re_k, 0);
+    for (int l = 0; l < 4; ++l) r.d[l] = div_any(EXACT ? a.d[l] - r.v * 0.0 : a.d[l], m.re, m.re_y, m.re_k, 0);
     return r;
   } else {
     return a / T(m.re);
   }
+}
+
+__device__ __forceinline__ bool not_finite(double v) {
+  return ((unsigned)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u;
 }
 
 // where a stencil's three results go
@@ -348,16 +360,16 @@ __device__ __forceinline__ bool mom_smooth(const DevBlock& B, int i, int j, int 
 // One fluid cell (i,j,k) of nsMomentum2order.  T = double: the reference
 // arithmetic (bit-exact drop-in).  T = float: the FP32 momentum stencil of the
 // mixed-precision path (fields stay FP64 in HBM; stencil values are rounded to
-// FP32 on load, ut/vt/wt stored back as FP64).
-template <typename T, class Rd, class Out>
+// FP32 on load, ut/vt/wt stored back as FP64).  EXACT: see GridNum.
+template <typename T, bool EXACT = false, class Rd, class Out>
 __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& a, int i, int j, int k,
                                               int64_t c, const Rd& rd, const Out& out) {
-  using G = typename GridNum<T>::type;
+  using G = typename GridNum<T, EXACT>::type;
   const G Q25 = G(0.25), HALF = G(0.5), alpha = G(1.0);
   const Dims& d = B.d;
   const G deltat = G(a.dt);
   const int gy = mom_groups(d.NX), gz = gy + mom_groups(d.NY);
-  const MomAxis<T> AX(B, 0, i), AY(B, gy, j), AZ(B, gz, k);
+  const MomAxis<T, EXACT> AX(B, 0, i), AY(B, gy, j), AZ(B, gz, k);
   const int nx_var = d.nx, ny_var = d.ny, nz_var = d.nz;
   const int64_t SX = 1, SY = d.NX, SZ = (int64_t)d.NX * d.NY;
   {
@@ -463,7 +475,7 @@ __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& 
           AY.quot(MQ_C) * (AY.div(-u8, MD_HALF_R) + AY.div(u6, MD_HALF_L));
       const auto d2udz2 =
           AZ.quot(MQ_C) * (AZ.div(-u12, MD_HALF_R) + AZ.div(u10, MD_HALF_L));
-      const auto xtt2 = div_re(d2udx2 + d2udy2 + d2udz2, a);
+      const auto xtt2 = div_re<EXACT>(d2udx2 + d2udy2 + d2udz2, a);
       const auto residu = (-duudx - dvudy - dwudz + xtt2);
       out.put(0, c, u(0, 0, 0) + deltat * (residu + dpdx));
     }
@@ -498,7 +510,7 @@ __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& 
       const auto d2vdy2 = AY.quot(MQ_2) * (AY.div(-v10, MD_R) + AY.div(v8, MD_D));
       const auto d2vdz2 =
           AZ.quot(MQ_C) * (AZ.div(-v14, MD_HALF_R) + AZ.div(v12, MD_HALF_L));
-      const auto ytt2 = div_re(d2vdx2 + d2vdy2 + d2vdz2, a);
+      const auto ytt2 = div_re<EXACT>(d2vdx2 + d2vdy2 + d2vdz2, a);
       const auto residv = (-duvdx - dvvdy - dwvdz + ytt2);
       out.put(1, c, v(0, 0, 0) + deltat * (residv + dpdy));
     }
@@ -533,7 +545,7 @@ __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& 
       const auto d2wdy2 =
           AY.quot(MQ_C) * (AY.div(-w12, MD_HALF_R) + AY.div(w10, MD_HALF_L));
       const auto d2wdz2 = AZ.quot(MQ_2) * (AZ.div(-w16, MD_R) + AZ.div(w14, MD_D));
-      const auto ztt2 = div_re(d2wdx2 + d2wdy2 + d2wdz2, a);
+      const auto ztt2 = div_re<EXACT>(d2wdx2 + d2wdy2 + d2wdz2, a);
       const auto residw = (-duwdx - dvwdy - dwwdz + ztt2);
       out.put(2, c, w(0, 0, 0) + deltat * (residw + dpdz));
     }
@@ -840,6 +852,16 @@ struct DualReader {
   }
 };
 
+// DualOut that notes whether a value is not finite
+struct DualOutChecked {
+  DualOut o;
+  bool* bad;
+  __device__ __forceinline__ void put(int q, int64_t c, Dual val) const {
+    o.put(q, c, val);
+    *bad |= not_finite(val.v);
+  }
+};
+
 struct MomentumTlmOp {
   MomArgs a;
   const double* du[4];
@@ -854,7 +876,9 @@ struct MomentumTlmOp {
         set_err(B.err, BCFD_E_STATE);  // the thin-surface overlay has no tangent model
         continue;
       }
-      momentum_cell<Dual>(B, a, i, j, k, c, rd, out);
+      bool bad = false;
+      momentum_cell<Dual>(B, a, i, j, k, c, rd, DualOutChecked{out, &bad});
+      if (bad) momentum_cell<Dual, true>(B, a, i, j, k, c, rd, out);
     }
   }
 };
@@ -887,9 +911,6 @@ struct FootReader {
     return __ldg(f[q] + x);
   }
 };
-__device__ __forceinline__ bool not_finite(double v) {
-  return ((unsigned)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u;
-}
 struct FiniteOut {  // whether an output is not finite
   bool* bad;
   __device__ __forceinline__ void put(int, int64_t, double v) const { *bad |= not_finite(v); }
@@ -1140,11 +1161,13 @@ __global__ void __launch_bounds__(128) k_mom_adjoint_static(DevBlock B, MomArgs 
   }
 }
 
-// The points that k_mom_adjoint_static leaves out.
+// The points that k_mom_adjoint_static leaves out: those that cells near TS
+// cells read, or (EXACT) all of them when a seed or an output is not finite.
 // One dual evaluation per (point, footprint offset) gives the partials of all
 // four fields at that point; each field's sum takes the offsets in ascending
 // order and, within one, the outputs U, V, W: the order of one evaluation per
 // field and offset, so the sums are those of four single-seed gathers.
+template <bool EXACT>
 __global__ void __launch_bounds__(128) k_mom_adjoint(DevBlock B, MomArgs a, const uint32_t* __restrict__ foot,
                                                      const double* ubar_t, const double* vbar_t,
                                                      const double* wbar_t, double* ub, double* vb, double* wb,
@@ -1152,8 +1175,8 @@ __global__ void __launch_bounds__(128) k_mom_adjoint(DevBlock B, MomArgs a, cons
   const Dims& d = B.d;
   const int64_t n = d.npts();
   const int nts = (int)min(B.cnt[C_TS], (int64_t)B.cap_ib);
-  const bool all = (__ldg(foot + 3) & kFootNonFinite) != 0, ts = B.cnt[C_TS] != 0;
-  if (!all && !ts) return;
+  if (((__ldg(foot + 3) & kFootNonFinite) != 0) != EXACT) return;
+  if (!EXACT && B.cnt[C_TS] == 0) return;
   double rc[N_KIND];
   restore_consts(B, nts, rc);
   uint32_t m[kFootWords];
@@ -1163,7 +1186,7 @@ __global__ void __launch_bounds__(128) k_mom_adjoint(DevBlock B, MomArgs a, cons
     const int xi = 1 + (int)(x % d.NX);
     const int64_t r = x / d.NX;
     const int xj = 1 + (int)(r % d.NY), xk = 1 + (int)(r / d.NY);
-    if (!all && !any_near_ts(B, xi, xj, xk, FootOffsets{})) continue;
+    if (!EXACT && !any_near_ts(B, xi, xj, xk, FootOffsets{})) continue;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (int o = 0; o < 125; ++o) {
       unsigned fmask = 0u;
@@ -1180,11 +1203,11 @@ __global__ void __launch_bounds__(128) k_mom_adjoint(DevBlock B, MomArgs a, cons
           continue;
         }
         const TsSeedReader4 rd{&B, ci, cj, ck, c, ts_last + N_KIND * c, rc, x};
-        momentum_cell<Dual4>(B, a, ci, cj, ck, c, rd, AdjOut4{{ubar_t, vbar_t, wbar_t}, acc, fmask});
+        momentum_cell<Dual4, EXACT>(B, a, ci, cj, ck, c, rd, AdjOut4{{ubar_t, vbar_t, wbar_t}, acc, fmask});
         continue;
       }
       const SeedReader4 rd{{B.u, B.v, B.w, B.p}, x};
-      momentum_cell<Dual4>(B, a, ci, cj, ck, c, rd, AdjOut4{{ubar_t, vbar_t, wbar_t}, acc, fmask});
+      momentum_cell<Dual4, EXACT>(B, a, ci, cj, ck, c, rd, AdjOut4{{ubar_t, vbar_t, wbar_t}, acc, fmask});
     }
     ub[x] += acc[0];
     vb[x] += acc[1];
@@ -1253,9 +1276,13 @@ __global__ void k_ts_last(DevBlock B, int* last) {
 }
 
 // per fluid cell near TS cells: seed . dF/d(scalar s) for its 14 scalars
-__global__ void __launch_bounds__(128) k_mom_ghost_contrib(DevBlock B, MomArgs a, const int* last,
+// (EXACT: when a seed or an output is not finite)
+template <bool EXACT>
+__global__ void __launch_bounds__(128) k_mom_ghost_contrib(DevBlock B, MomArgs a, const uint32_t* __restrict__ foot,
+                                                           const int* last,
                                                            const double* ubar_t, const double* vbar_t,
                                                            const double* wbar_t, double* contrib) {
+  if (((__ldg(foot + 3) & kFootNonFinite) != 0) != EXACT) return;
   const Dims& d = B.d;
   const int nts = (int)min(B.cnt[C_TS], (int64_t)B.cap_ib);
   double rc[N_KIND];
@@ -1270,7 +1297,7 @@ __global__ void __launch_bounds__(128) k_mom_ghost_contrib(DevBlock B, MomArgs a
     for (int pass = 0; pass < 4; ++pass) {
       double acc[4] = {0.0, 0.0, 0.0, 0.0};
       const TsGhostReader4 rd{&B, i, j, k, c, last + N_KIND * c, rc, pass};
-      momentum_cell<Dual4>(B, a, i, j, k, c, rd, AdjOut4{{ubar_t, vbar_t, wbar_t}, acc, 0xFu});
+      momentum_cell<Dual4, EXACT>(B, a, i, j, k, c, rd, AdjOut4{{ubar_t, vbar_t, wbar_t}, acc, 0xFu});
 #pragma unroll
       for (int l = 0; l < 4; ++l)
         if (4 * pass + l < 2 * N_KIND) contrib[2 * N_KIND * c + 4 * pass + l] = acc[l];
@@ -1615,13 +1642,18 @@ int launch_momentum_adjoint(HostBlock* hb, double dt, double re, const double* c
   k_mom_adjoint_static<<<grid_for(hb->d.d.npts(), 128, 1u << 20), 128, 0, stream()>>>(
       hb->d, a, foot, sb[0], sb[1], sb[2], ab[0], ab[1], ab[2], ab[3]);
   BCFD_LAUNCHED();
-  k_mom_adjoint<<<grid_for(hb->d.d.npts(), 128, 1u << 20), 128, 0, stream()>>>(
-      hb->d, a, foot, sb[0], sb[1], sb[2], ab[0], ab[1], ab[2], ab[3], last);
-  BCFD_LAUNCHED();
-  if (ts) {
-    k_mom_ghost_contrib<<<grid_for(ni, 128, 1u << 16), 128, 0, stream()>>>(hb->d, a, ts->last, sb[0], sb[1], sb[2],
-                                                                           ts->contrib);
+  // of each pair below one returns at once: what is not finite is known on the
+  // device only
+  for (const auto fn : {k_mom_adjoint<false>, k_mom_adjoint<true>}) {
+    fn<<<grid_for(hb->d.d.npts(), 128, 1u << 20), 128, 0, stream()>>>(hb->d, a, foot, sb[0], sb[1], sb[2], ab[0],
+                                                                      ab[1], ab[2], ab[3], last);
     BCFD_LAUNCHED();
+  }
+  if (ts) {
+    for (const auto fn : {k_mom_ghost_contrib<false>, k_mom_ghost_contrib<true>}) {
+      fn<<<grid_for(ni, 128, 1u << 16), 128, 0, stream()>>>(hb->d, a, foot, ts->last, sb[0], sb[1], sb[2], ts->contrib);
+      BCFD_LAUNCHED();
+    }
     k_mom_ghost_acc<<<1, 32, 0, stream()>>>(hb->d, ts->last, ts->contrib, ts->gb, ts->cap);
     BCFD_LAUNCHED();
   }
