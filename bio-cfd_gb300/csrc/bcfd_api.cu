@@ -108,11 +108,12 @@ namespace {
 __global__ void k_wait_unreachable(GridBar gb) { (void)grid_sync(gb); }
 }  // namespace
 
-GridBar make_bar(int* err, unsigned nblocks) {
+GridBar make_bar(int* err, unsigned nblocks, bool heed) {
   GridBar g{};
   g.err = err;
   g.nblocks = nblocks;
   g.limit_ns = lib().wait_limit_ns;
+  g.heed = heed;
   return g;
 }
 

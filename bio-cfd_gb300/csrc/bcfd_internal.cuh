@@ -194,11 +194,17 @@ __device__ inline void set_err(int* err, int code) { atomicCAS(err, 0, code); }
 // counter (zeroed before the launch).  The k-th barrier completes when the
 // counter reaches k * nblocks; bit 63 set means "abandon": a CTA that gave up
 // (timeout or a recorded error) sets it so every waiter leaves at once.
+// With `heed` a wait of 64 polls or more also gives up when `err` holds an
+// error.  A kernel whose CTAs leave only through the abandon bit or at the end
+// runs without it: an error that an earlier launch of the step recorded (a
+// NaN, a probe without a bracket) is no reason to drop its work, and whether
+// the work is dropped would hang on how long a wait happens to take.
 struct GridBar {
   unsigned long long* ctr;
   int* err;          // set to BCFD_E_TIMEOUT when a wait exceeds the limit
   unsigned nblocks;
   unsigned long long limit_ns;  // longest a single wait may last
+  bool heed;
 };
 constexpr unsigned long long kBarAbandon = 1ull << 63;
 
@@ -265,7 +271,7 @@ __device__ inline bool grid_sync(const GridBar& gb) {
         if (v & kBarAbandon) { ok = 0; break; }
         if (v >= target) break;
         if (((++spins) & 63u) == 0) {
-          if (ld_acquire_i(gb.err) != 0) {
+          if (gb.heed && ld_acquire_i(gb.err) != 0) {
             atomicOr(gb.ctr, kBarAbandon);
             ok = 0;
             break;
@@ -338,6 +344,6 @@ cudaError_t launch_coop(const void* fn, unsigned grid, unsigned block, void** ar
 unsigned coop_grid(const void* fn, int threads, size_t smem, unsigned want);
 
 // barrier state for persistent kernels (owned by the library)
-GridBar make_bar(int* err, unsigned nblocks);
+GridBar make_bar(int* err, unsigned nblocks, bool heed = true);
 
 }  // namespace bcfd

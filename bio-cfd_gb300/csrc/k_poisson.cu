@@ -1697,7 +1697,7 @@ __device__ __forceinline__ bool res_import(const DevBlock& B, const ResTile& R, 
       if (!more) break;
       if ((++spins & 63u) == 0) {
         if (t0 == 0) t0 = globaltimer_ns();
-        if ((ld_relaxed_u64(gb.ctr) & kBarAbandon) || ld_acquire_i(gb.err) != 0) return false;
+        if (ld_relaxed_u64(gb.ctr) & kBarAbandon) return false;
         if (globaltimer_ns() - t0 > gb.limit_ns) {
           atomicCAS(gb.err, 0, BCFD_E_TIMEOUT);
           return false;
@@ -2024,7 +2024,7 @@ __device__ __forceinline__ bool res64_import(const DevBlock& B, const Res64Tile&
       if (!more) break;
       if ((++spins & 63u) == 0) {
         if (t0 == 0) t0 = globaltimer_ns();
-        if ((ld_relaxed_u64(gb.ctr) & kBarAbandon) || ld_acquire_i(gb.err) != 0) return false;
+        if (ld_relaxed_u64(gb.ctr) & kBarAbandon) return false;
         if (globaltimer_ns() - t0 > gb.limit_ns) {
           atomicCAS(gb.err, 0, BCFD_E_TIMEOUT);
           return false;
@@ -2705,7 +2705,7 @@ static int launch_sor64_res(HostBlock* hb, SorArgs a) {
   TRY_R(reset_solve_state(hb, TileMap{z.tj, z.tk, z.ntj, z.ntk, hb->prog, 1}));
   BCFD_CUDA(cudaFuncSetAttribute((const void*)k_sor64_res, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const unsigned grid = (unsigned)(z.ntj * z.ntk);
-  GridBar gb = make_bar(B.err, grid);
+  GridBar gb = make_bar(B.err, grid, false);
   gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
   void* args[] = {(void*)&B, (void*)&a, (void*)&gb, (void*)&z};
   prof_mark(true);
@@ -3007,7 +3007,7 @@ static int launch_sor_res(HostBlock* hb, int64_t itmax, double dt, double div_to
   BCFD_CUDA(cudaFuncSetAttribute((const void*)k_sor_res, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   DcArgs a = mixed_args(hb, itmax, dt, div_tol);
   const unsigned grid = (unsigned)(z.ntj * z.ntk);
-  GridBar gb = make_bar(B.err, grid);
+  GridBar gb = make_bar(B.err, grid, false);
   gb.ctr = reinterpret_cast<unsigned long long*>(hb->bar);
   void* args[] = {(void*)&B, (void*)&a, (void*)&gb, (void*)&z};
   prof_mark(true);
