@@ -1433,6 +1433,14 @@ int bcfd_profile_end(bcfd_profile_report* out) {
       // and the mask once and writes e once (4 + 4 + 1 + 4 B); the FP64
       // residual and update passes as below
       out->sor_bytes += 0.5 * sw * fl * 13.0 + rp * fl * 29.0 + (rp - 1.0) * fl * 25.0;
+    } else if (e[4 * q + 3] == 3) {
+      // resident FP32 sweeps: e, right-hand side and mask stay on the chip; a
+      // correction reads the residual once and updates pc (4 + 8 + 8 B)
+      out->sor_bytes += rp * fl * 29.0 + (rp - 1.0) * fl * 20.0;
+    } else if (e[4 * q + 3] == 4) {
+      // resident FP64 sweeps: b/dt and mask per pair (8 + 1 B), pc in and out
+      // once per solve
+      out->sor_bytes += sw * fl * 9.0 + fl * 16.0;
     } else {
       // FP32 sweeps 4w + 1 (w = 4); FP64 residual: pc own + neighbours + b/dt
       // read, r written as FP32, mask (8+8+8+4+1); update x += e: pc r/w,

@@ -175,7 +175,7 @@ struct BlockStats {
 enum CountSlot { C_IB = 0, C_SOLID, C_FLUID, C_RED, C_BLACK, C_TS, N_COUNT };
 
 // entries of the solve log of a measurement window ({sweeps, residual
-// passes, fluid cells, precision} each, after one counter word)
+// passes, fluid cells, kind of sweeps} each, after one counter word)
 constexpr unsigned long long kProfLogCap = 4096;
 // most CTAs (tiles) of a tiled persistent solve; each tile's phase counter
 // sits on its own 128-byte line (kTileStride unsigned words apart)

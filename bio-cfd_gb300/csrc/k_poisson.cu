@@ -425,9 +425,10 @@ struct SorArgs {
   int fast;       // 1: division-free update (not the reference's arithmetic)
 };
 
-// append {sweep pairs, FP64 residual passes, fluid cells, precision}
+// append {sweep pairs, FP64 residual passes, fluid cells, kind}; kind: 0 tiled
+// FP64, 1 tiled FP32, 2 z-marching FP32, 3 resident FP32, 4 resident FP64 sweeps
 __device__ __forceinline__ void log_solve(int64_t* log, int64_t sweeps, int64_t res_passes,
-                                          int64_t fluid, int64_t precision) {
+                                          int64_t fluid, int64_t kind) {
   if (!log) return;
   const unsigned long long s = atomicAdd(reinterpret_cast<unsigned long long*>(log), 1ull);
   if (s < kProfLogCap) {
@@ -435,7 +436,7 @@ __device__ __forceinline__ void log_solve(int64_t* log, int64_t sweeps, int64_t 
     e[0] = sweeps;
     e[1] = res_passes;
     e[2] = fluid;
-    e[3] = precision;
+    e[3] = kind;
   }
 }
 
@@ -1923,7 +1924,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sor_res(DevBlock B, DcArgs a
     if (!grid_sync(gb)) return;
   }
   if (cta == 0 && threadIdx.x == 0) {
-    log_solve(a.log, sweeps, outer + 1, B.cnt[C_FLUID], 1);
+    log_solve(a.log, sweeps, outer + 1, B.cnt[C_FLUID], 3);
     st->niter = st->niter + sweeps;
     st->derr2 = a.dt * res;
     st->pad[1] = a.dt * res;
@@ -2279,7 +2280,7 @@ __global__ void __launch_bounds__(kRes64Threads, 1) k_sor64_res(DevBlock B, SorA
     }
   }
   if (cta == 0 && threadIdx.x == 0) {
-    log_solve(a.log, it - it0, 0, B.cnt[C_FLUID], 0);
+    log_solve(a.log, it - it0, 0, B.cnt[C_FLUID], 4);
     st->niter = it;
     st->derr2 = derr4;
     if (ok && non_finite(derr4)) set_err(B.err, BCFD_E_NONFINITE);

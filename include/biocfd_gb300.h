@@ -463,8 +463,10 @@ typedef struct bcfd_profile_report {
   double sor_ms;          /* their summed device time (CUDA events, library stream) */
   double sor_bytes;       /* algorithmic bytes they moved (4w+1 B per cell sweep
                              pair, w = 8 FP64 / 4 FP32; 13 B per cell per two
-                             pairs for the z-marching sweeps; plus the FP64
-                             residual and update passes of the mixed solve)       */
+                             pairs for the z-marching sweeps; none for the
+                             resident FP32 and 9 B for the resident FP64 sweeps,
+                             whose tiles stay on the chip; plus the FP64 residual
+                             and update passes of the mixed solve)                */
   int64_t sor_sweeps;     /* red+black sweep pairs done by them                    */
   int64_t kernel_launches;/* kernels launched in the window                        */
 } bcfd_profile_report;
