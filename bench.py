@@ -497,13 +497,12 @@ def sweep_roofline(torch, local, hbm, block=(384, 256, 256), fp32_pairs=40, fp64
     cells = block[0] * block[1] * block[2]
     out = {"block": "x".join(map(str, block)) + f" ({cells / 1e6:.1f}M cells), no body",
            "l2": f"FP32 working set {17 * cells / 1e6:.0f} MB vs 129 MB L2", "solve_launch": s.solve_launch(g)}
-    tuned = s.solve_launch(g)
     for prec, pairs, key in ((1, fp32_pairs, "fp32"), (1, fp32_pairs, "fp32_tiled_neighbour_sync"),
                              (1, fp32_pairs, "fp32_zmarch_tma"), (0, fp64_pairs, "fp64_reference_sweeps"),
                              (2, fp64_pairs, "fp64_division_free")):
-        # fp32: the autotuned variant; then the tiled sweeps with neighbour
-        # sync (variant 3) and the z-marching TMA sweeps (variant 5) alone
-        variant = {"fp32": tuned["fp32_variant"], "fp32_tiled_neighbour_sync": 3, "fp32_zmarch_tma": 5}.get(key)
+        # fp32: as autotuned; then the tiled sweeps with neighbour sync
+        # (variant 3) and the z-marching TMA sweeps (variant 5) alone
+        variant = {"fp32_tiled_neighbour_sync": 3, "fp32_zmarch_tma": 5}.get(key)
         if variant is not None:
             s.set_mixed_params(variant=variant, block=g)
         runs = {}

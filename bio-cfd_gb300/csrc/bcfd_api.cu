@@ -1337,8 +1337,12 @@ int bcfd_block_set_solve_launch(bcfd_handle h, int threads, int ctas_per_sm, int
   LOCK();
   GETB(h);
   if (!(threads == 0 || threads == 128 || threads == 256 || threads == 512) ||
-      ctas_per_sm < 0 || ctas_per_sm > 16 || fp64_sync < 0 || fp64_sync > 1)
+      ctas_per_sm < 0 || ctas_per_sm > 16 || fp64_sync < 0 || fp64_sync > kSyncResident)
     return BCFD_E_ARG;
+  // the autotuner's resident sweeps are a launch shape: the one asked for
+  // replaces them, and variant 1, under which they are reported, goes with them
+  if (hb->dc_resident) hb->dc_variant = 0;
+  hb->dc_resident = false;
   hb->solve_threads = threads;
   hb->solve_ctas_per_sm = ctas_per_sm;
   hb->solve_sync = fp64_sync;
@@ -1371,6 +1375,9 @@ int bcfd_block_set_mixed_params(bcfd_handle h, int64_t inner_sweeps, double omeg
   if (inner_sweeps < 0 || inner_sweeps > 100000 || omega < 0.0 || omega >= 2.0 || variant < 0 || variant > 6 ||
       variant == 2)  // the cluster-resident variant was withdrawn
     return BCFD_E_ARG;
+  // likewise the thread count of the autotuner's resident sweeps
+  if (hb->dc_resident) hb->dc_threads = 0;
+  hb->dc_resident = false;
   hb->dc_inner = (int)inner_sweeps;
   hb->dc_omega = omega;
   hb->dc_variant = variant;

@@ -125,6 +125,9 @@ struct HostBlock {
   int sor_rev = 0;                 // FP64 solve: black half-sweep first (adjoint solves)
   int dc_threads = 0;              // FP32 correction: threads per CTA (0: 256)
   int dc_ctas_per_sm = 0;          // FP32 correction: CTAs per SM cap (0: occupancy limit)
+  // the autotuner chose the resident FP32 sweeps, reported as variant 1 with
+  // kResThreads threads; a variant or launch shape asked for replaces the choice
+  bool dc_resident = false;
   // largest distance of a surface node from the block centre (for the FP32
   // prefilter bound of the nearest-element search)
   double node_rmax = 0.0;
@@ -271,6 +274,8 @@ bool zm_solve_fits(HostBlock* hb);
 bool res_solve_fits(HostBlock* hb);
 bool res64_solve_fits(HostBlock* hb);
 constexpr int kSyncResident = 2;  // HostBlock::solve_sync of the resident FP64 solve
+constexpr int kVariantResident = 6;  // bcfd_block_set_mixed_params' variant of the resident FP32 sweeps
+constexpr int kResThreads = 512;  // most threads of their CTAs
 double mixed_omega_of(const HostBlock* hb);
 int launch_sor_mixed_set(const std::vector<HostBlock*>& hbs, int64_t itmax, double dt, double div_tol);
 // res_tol > 0: stop on the FP64 residual dt*max|b/dt - A pc| <= res_tol

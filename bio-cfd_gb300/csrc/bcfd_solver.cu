@@ -511,9 +511,9 @@ std::vector<unsigned char> step_key(const bcfd_step_config& c) {
     const unsigned char none = 0;
     if (!hb) { put(&none, 1); continue; }
     put(&hb->d, sizeof hb->d);
-    const int sw[11] = {hb->is_coarse, hb->has_body, (int)hb->move_check, (int)hb->blk_mv_tag, hb->dc_inner,
+    const int sw[12] = {hb->is_coarse, hb->has_body, (int)hb->move_check, (int)hb->blk_mv_tag, hb->dc_inner,
                         hb->dc_variant, hb->solve_threads, hb->solve_ctas_per_sm, hb->solve_sync,
-                        hb->dc_threads, hb->dc_ctas_per_sm};
+                        hb->dc_threads, hb->dc_ctas_per_sm, hb->dc_resident};
     put(sw, sizeof sw);
     put(&hb->dc_omega, sizeof hb->dc_omega);
     put(&hb->omega, sizeof hb->omega);

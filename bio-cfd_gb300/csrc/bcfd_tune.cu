@@ -23,7 +23,7 @@ namespace {
 
 struct Shape {
   int threads, ctas_per_sm, sync;  // sync: FP64 0 neighbour / 1 grid / 2 resident; FP32 variant 1 grid / 3 neighbour,
-                                   // 4 temporal-blocked, 5 z-marching TMA
+                                   // 4 temporal-blocked, 5 z-marching TMA, 6 resident
 };
 struct Tuned {
   Shape fp64, fp32;
@@ -139,7 +139,8 @@ void apply(HostBlock* hb, const Shape& s, bool fp32) {
   if (fp32) {
     hb->dc_threads = s.threads;
     hb->dc_ctas_per_sm = s.ctas_per_sm;
-    hb->dc_variant = s.sync;
+    hb->dc_resident = s.sync == kVariantResident;
+    hb->dc_variant = hb->dc_resident ? 1 : s.sync;
   } else {
     hb->solve_threads = s.threads;
     hb->solve_ctas_per_sm = s.ctas_per_sm;
@@ -153,9 +154,9 @@ int tune_block(HostBlock* hb, Tuned* out) {
   // {256, 4, *} selects the 64-register instantiation of the FP32 solve
   // {512, 0, 4}: the temporal-blocked sweeps (small blocks)
   // {384, 0, 5}: the z-marching TMA sweeps (large blocks)
-  // {512, 0, 1}: the resident sweeps (blocks that fit the SMs' shared memory)
+  // {512, 0, 6}: the resident sweeps (blocks that fit the SMs' shared memory)
   static const Shape c32[] = {{128, 0, 1}, {256, 0, 1}, {128, 0, 3}, {256, 0, 3}, {256, 2, 1},
-                              {256, 1, 1}, {256, 4, 1}, {256, 4, 3}, {512, 0, 4}, {384, 0, 5}, {512, 0, 1}};
+                              {256, 1, 1}, {256, 4, 1}, {256, 4, 3}, {512, 0, 4}, {384, 0, 5}, {kResThreads, 0, kVariantResident}};
   Saved sv;
   if (const int e = save_state(hb, sv, false)) {
     cudaFree(sv.buf);
@@ -163,6 +164,7 @@ int tune_block(HostBlock* hb, Tuned* out) {
   }
   const int t0 = hb->solve_threads, c0 = hb->solve_ctas_per_sm, s0 = hb->solve_sync, v0 = hb->dc_variant,
             dt0 = hb->dc_threads, dc0 = hb->dc_ctas_per_sm;
+  const bool res0 = hb->dc_resident;
   int r = 0;
   float best = 1e30f, best64 = 1e30f;
   Shape b64 = c64[0], b32 = c32[0];
@@ -179,7 +181,7 @@ int tune_block(HostBlock* hb, Tuned* out) {
     if (r) break;
     if (s.sync == 4 && !tb_solve_fits(hb)) continue;
     if (s.sync == 5 && !zm_solve_fits(hb)) continue;
-    if (s.sync == 1 && s.threads == 512 && !res_solve_fits(hb)) continue;
+    if (s.sync == kVariantResident && !res_solve_fits(hb)) continue;
     apply(hb, s, true);
     float ms = 0;
     if ((r = time_trial(hb, true, 16, &ms))) break;
@@ -191,6 +193,7 @@ int tune_block(HostBlock* hb, Tuned* out) {
   hb->dc_variant = v0;
   hb->dc_threads = dt0;
   hb->dc_ctas_per_sm = dc0;
+  hb->dc_resident = res0;
   const int rr = save_state(hb, sv, true);
   cudaStreamSynchronize(stream());
   cudaFree(sv.buf);

@@ -1524,8 +1524,6 @@ __global__ void __launch_bounds__(kZmThreads, 1) k_sor_zm(DevBlock B, DcArgs a, 
 // keeps one run position a, so the x coefficients stay in registers over its
 // rows.
 // ---------------------------------------------------------------------------
-constexpr int kResThreads = 512;
-
 struct ResArgs {
   int tj, tk, ntj, ntk;
   int half;                   // threads per parity group (blockDim.x == 2 * half)
@@ -3026,9 +3024,8 @@ int launch_sor_mixed(HostBlock* hb, int64_t itmax, double dt, double div_tol) {
   // wherever they fit: on every such size measured they are faster than the
   // tiled ones, 4.64 -> 1.47 us per sweep pair on 33x21x27, 5.2 -> 2.4 on 64^3,
   // 8.2 -> 5.0 on 128x96x96, 10.3 -> 6.7 on 128^3
-  // (the autotuner names them variant 1 with kResThreads threads)
   const bool shaped = hb->dc_variant != 0 || hb->dc_threads > 0 || hb->dc_ctas_per_sm > 0;
-  if ((hb->dc_variant == 6 || !shaped || (hb->dc_variant == 1 && hb->dc_threads == kResThreads)) && res_solve_fits(hb))
+  if ((hb->dc_variant == kVariantResident || hb->dc_resident || !shaped) && res_solve_fits(hb))
     return launch_sor_res(hb, itmax, dt, div_tol);
   for (int c = 0; c < 2; ++c) BCFD_CUDA(cudaMemsetAsync(B.pcf[c], 0, np * sizeof(float), stream()));
   if (hb->dc_variant == 4 && tb_solve_fits(hb)) return launch_sor_tb(hb, itmax, dt, div_tol);

@@ -421,7 +421,9 @@ int bcfd_block_get_divergence(bcfd_handle h, double* out);
  * resident sweeps, each SM keeping a tile of the correction in shared memory,
  * when the block fits the SMs' shared memory, else 1; all of them give bitwise
  * the same corrections; 2 is not accepted).  The library's choice is 6 where
- * it fits, else 1 */
+ * it fits and the block is solved in a launch of its own; 1 elsewhere, among
+ * others for the untuned blocks that batching solves side by side in one
+ * launch */
 int bcfd_block_set_mixed_params(bcfd_handle h, int64_t inner_sweeps, double omega, int variant);
 /* the relaxation factor block h's FP32 correction sweeps use (its setting or
  * the default: 2 / (1 + sqrt(1 - rho^2)), rho = (cos(pi/nx) + cos(pi/ny) +
@@ -432,12 +434,17 @@ int bcfd_block_get_mixed_omega(bcfd_handle h, double* omega);
  * effect on results): threads per CTA (0 = the default: 256 for the FP64
  * solve, 256 for the mixed one, which takes at most 256; else 128/256/512), cap
  * on co-resident CTAs per SM (0 = occupancy limit), and the FP64 solve's
- * phase sync (0 point-to-point between neighbour tiles, 1 grid-wide) */
+ * phase sync (0 point-to-point between neighbour tiles, 1 grid-wide, 2: the
+ * resident solve, each SM keeping a tile of pc in shared memory, when the block
+ * fits the SMs' shared memory, else 0; threads and cap do not apply to it).
+ * With 0, 0, 0 the library chooses: resident for a block of up to 200,000
+ * cells that is solved in a launch of its own, else point-to-point */
 int bcfd_block_set_solve_launch(bcfd_handle h, int threads, int ctas_per_sm, int fp64_sync);
-/* out[6] = FP64 solve threads, CTAs/SM cap, sync (2: the resident solve, each
- * SM keeping a tile of pc in shared memory); FP32 correction threads,
- * CTAs/SM cap, variant (0 = library default; 1 with 512 threads: the resident
- * sweeps) */
+/* out[6] = FP64 solve threads, CTAs/SM cap, sync; FP32 correction threads,
+ * CTAs/SM cap, variant (0 = library default).  An autotuner's choice of the
+ * resident FP32 sweeps reads as variant 1 with 512 threads, a count that cannot
+ * be asked for; bcfd_block_set_mixed_params (variant 6 asks for the same) and
+ * bcfd_block_set_solve_launch replace it */
 int bcfd_block_get_solve_launch(bcfd_handle h, int* out);
 /* Autotuner (no counterpart in the reference): for every block, times short
  * solves under each candidate launch shape of the FP64 solve and of the FP32
