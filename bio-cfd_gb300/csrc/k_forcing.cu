@@ -631,7 +631,7 @@ __global__ void k_p_ghost(DevBlock B) {
 // was overwritten), add coefficient x adjoint to each stencil point.  A read
 // of a value an earlier task wrote becomes an add that the earlier task picks
 // up when its turn comes, which is exactly the chain rule through the serial
-// order.  One thread runs the reverse sweep, so the sums have a fixed order.
+// order.  One warp runs the reverse sweep, so the sums have a fixed order.
 // ---------------------------------------------------------------------------
 __global__ void k_force_coef(DevBlock B, int mode, int vel, ForceCoef fc) {
   const int nib = (int)min(B.cnt[mode == 2 ? C_TS : C_IB], (int64_t)B.cap_ib);

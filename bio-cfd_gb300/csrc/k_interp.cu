@@ -356,9 +356,10 @@ FaceArgs make_args(HostInterface* it, HostBlock* a, HostBlock* b, int comp) {
 }  // namespace
 
 
-// the face fill of several components: one launch per face pass (the
-// components write different arrays and read the coarse block only; the
-// passes keep their order, so points two passes write get the later value)
+// the face fill of several components and the three face passes in one launch:
+// they read the coarse block only, the components write different arrays, and a
+// point that two passes write gets the same value from both (it belongs to one
+// entry triple), so they need no order
 int launch_face_fill_set(HostInterface* it, const int* comps, int nc, int which) {
   HostBlock* a = get_block(it->a);
   HostBlock* b = get_block(it->b);

@@ -358,9 +358,10 @@ __device__ __forceinline__ bool mom_smooth(const DevBlock& B, int i, int j, int 
 }
 
 // One fluid cell (i,j,k) of nsMomentum2order.  T = double: the reference
-// arithmetic (bit-exact drop-in).  T = float: the FP32 momentum stencil of the
-// mixed-precision path (fields stay FP64 in HBM; stencil values are rounded to
-// FP32 on load, ut/vt/wt stored back as FP64).  EXACT: see GridNum.
+// arithmetic (bit-exact drop-in).  T = FastF or float: the FP32 momentum stencil
+// of the mixed-precision path (it reads the fields' FP32 copies, beside
+// thin-surface cells the FP64 fields rounded on load; ut/vt/wt are stored as
+// FP64).  EXACT: see GridNum.
 template <typename T, bool EXACT = false, class Rd, class Out>
 __device__ __forceinline__ void momentum_cell(const DevBlock& B, const MomArgs& a, int i, int j, int k,
                                               int64_t c, const Rd& rd, const Out& out) {

@@ -1629,8 +1629,8 @@ __device__ __forceinline__ void res_segments(const DevBlock& B, const ResTile& R
   }
 }
 
-// the halo rows of pair `pair` into shared memory; all of a thread's first
-// four runs' loads are in flight together.  false: the wait gave up
+// the halo rows of pair `pair` into shared memory; the loads of U of a thread's
+// runs are in flight together.  false: the wait gave up
 __device__ __forceinline__ bool res_import(const DevBlock& B, const ResTile& R, const unsigned* list, int n,
                                            const unsigned long long* ll, unsigned pair, const GridBar& gb) {
   constexpr int U = 2;

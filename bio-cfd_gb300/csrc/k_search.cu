@@ -107,7 +107,7 @@ __device__ void warp_nearest(const QueryCtx& C, const double (&q)[Q][3], int (&o
   // one chunk: every query's minimum over its elements (warp-uniform result)
   // by one reduction of the bit patterns (distances are not negative: ordered
   // as integers, NaN above all) instead of five exchanges per query and chunk,
-  // the chain that bounds a query: moved 160x144x96 plate 2.55 -> 2.45 ms
+  // the chain that bounds a query: moved 160x144x96 plate 2.55 -> 2.47 ms
   auto visit1 = [&](int c) {
     const int pos = 32 * c + lane;
     float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
