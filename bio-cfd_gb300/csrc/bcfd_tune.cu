@@ -149,8 +149,8 @@ void apply(HostBlock* hb, const Shape& s, bool fp32) {
 }
 
 int tune_block(HostBlock* hb, Tuned* out) {
-  // sync 2: the resident solve
-  static const Shape c64[] = {{256, 0, 0}, {512, 0, 0}, {256, 0, 1}, {512, 0, 1}, {512, 1, 0}, {512, 0, kSyncResident}};
+  // sync 2: the resident solve; 512 threads are one CTA per SM without a cap too
+  static const Shape c64[] = {{256, 0, 0}, {512, 0, 0}, {256, 0, 1}, {512, 0, 1}, {512, 0, kSyncResident}};
   // {256, 4, *} selects the 64-register instantiation of the FP32 solve
   // {512, 0, 4}: the temporal-blocked sweeps (small blocks)
   // {384, 0, 5}: the z-marching TMA sweeps (large blocks)
